@@ -6,7 +6,7 @@
 // p = t % 128 and the half h = t / 128 of the harmonics (and the same TMEM
 // lane p in the tensor-core epilogues). Per tile:
 //   1  stage the rotated body points of the pairs in shared memory;
-//   2  descriptor forward (FP32): g = [sum_a f_n(a) | sum_m A_{n,lm}^2];
+//   2  descriptor forward (FP32): g = [sum_a f_n(a) | sum_m N_lm^2 A_{n,lm}^2];
 //   3  net forward and backward on the tensor cores: every product is three
 //      bf16 x bf16 -> fp32 MMAs (hi*hi + hi*lo + lo*hi of the bf16 splits of
 //      activations and weights), accumulators in TMEM; gives dE/dg;
@@ -33,8 +33,13 @@ __device__ int g_amlp_first_wait_limit = -1;
 
 namespace {
 
-constexpr int kAP = 128;          // pairs per tile (MMA M)
-constexpr int kAThreads = 256;
+constexpr int kAP = 128;          // pairs per tile of the fused kernel (MMA M)
+constexpr int kAThreads = 2 * kAP;
+// Pairs per tile of the wide path's descriptor kernels: two CTAs of 64 pairs on an
+// SM, so that one's loads, staging and scatter run under the other's point loops
+// (backward 1,376 -> 1,222 us at 60,001 cylinders against one CTA of 128).
+constexpr int kDP = 64;
+constexpr int kDThreads = 2 * kDP;
 constexpr int kMaxHidden = 3;      // hidden layers of the fused kernel
 constexpr int kMaxHiddenWide = 4;  // hidden layers of the wide path: layer_first + 3 (TheEnergyNet(150, 3, D))
 constexpr int kWpad = 64;          // hidden widths padded to 64 in TMEM regions
@@ -82,81 +87,119 @@ __device__ __forceinline__ void act_pair(int act, float z, float &f, float &df) 
     }
 }
 
-// Radial basis f_n of the adjoint kernels, with the cutoff function from the
-// hardware sine/cosine (__sincosf: a few 1e-7 absolute error for the
-// arguments here, far below the tensor-core net's 1e-5), used by both their
-// forward and their backward so that the forces stay the exact derivative of
-// the energy they compute.
-template <int NR>
-__device__ __forceinline__ void radial_basis_fast(float d, float inv_rc, float *f) {
-    const float u = d * inv_rc, um1 = u - 1.0f;
-    const float x = fmaf(2.0f * um1, um1, -1.0f);
-    float s, c;
-    __sincosf(3.14159265358979f * u, &s, &c);
-    const float hfc = fmaf(0.25f, c, 0.25f);  // fc / 2
-    float tm1 = 1.0f, t = x;
-    f[0] = 2.0f * hfc;
-    if (NR > 1) f[1] = fmaf(hfc, x, hfc);
-#pragma unroll
-    for (int n = 2; n < NR; ++n) {
-        const float tn = fmaf(2.0f * x, t, -tm1);
-        tm1 = t;
-        t = tn;
-        f[n] = fmaf(hfc, tn, hfc);
-    }
+// ---------------------------------------------------------------- harmonic halves
+// The 24 harmonics of l = 1..4 split over the two threads of a pair by order m,
+// twelve each: half 0 holds m = 0 and 1, half 1 holds m = 2, 3 and 4. Half 0 needs
+// the polynomials in z and x, y themselves, half 1 the powers
+// C_m + i S_m = (x + i y)^m and few polynomials, so neither runs recurrences that
+// only the other uses, and both take about the same time. Split by index (l = 1, 2
+// and part of 3 | the rest), half 1 ran every recurrence up to l = m = 4 while
+// half 0's warps waited at the barrier.
+//
+// The radial functions are f_n = h (1 + T_n(x)) with h = fc / 2. The backward
+// holds, per harmonic, the coefficients of q_k(x) = sum_n G_nk (1 + T_n(x)) in
+// the basis 1, T_1, .., T_8, and forms neither f_n nor f_n' per point. Its
+// harmonics carry the scale that makes their derivatives come out of the same
+// few polynomials, with c3 = 5 z^2 - 1, c4 = z (7 z^2 - 3), c7 = 7 z^2 - 1:
+//   m = 0: z, z^2/2 - 1/6, 5/3 z^3 - z, 7/4 z^4 - 3/2 z^2 + 3/20  (d/dz: 1, z, c3, c4)
+//   m = 1: {x, y} times 1, z, c3, c4      (d/dz of the last three: 1, 10 z, 21 z^2 - 3)
+//   m = 2: {C_2, S_2} times 1, z, c7      (d/dz: 0, 1, 14 z)
+//   m = 3: {C_3, S_3} times 1, z;  m = 4: {C_4, S_4}
+// The sums over harmonics run on pairs of them (fma.rn.f32x2): two multiply-adds
+// per instruction at the same rate, which keeps the unrolled loops half as long
+// (4.30 -> 4.17 ms at 131,072 cubes).
+//
+// Both loops are bound by instruction issue: a multiply-add of the 9 x 24 sums
+// (108 per point and half forward, 204 backward) comes with about as many other
+// instructions. Measured with these changes: the fused kernel 5.02 -> 4.20 ms at
+// 131,072 cubes; at 60,001 cylinders the descriptor forward 751 -> 617 us and the
+// backward 1,594 -> 1,160 us. Slower, so not kept: three threads per pair (twelve
+// warps, 4.99 ms), two teams of 64 pairs per CTA in the fused kernel (4.66 ms), the
+// next point's distance and radial functions one iteration ahead.
+constexpr int kHalfK = 12;  // harmonics per half
+constexpr int kHalfP = kHalfK / 2;
+// Points per iteration of the forward's loop: four overlap one point's chain
+// (load, square root, cosine, recurrences) with another's sums, 669 -> 617 us at
+// 60,001 cylinders; the fused kernel, whose code is longer, is faster with one
+// (4.20 against 4.23 ms at 131,072 cubes). The backward takes two (1,203 -> 1,160 us,
+// 4.27 -> 4.23 ms).
+constexpr int kWideUnroll = 4, kFusedUnroll = 1, kBackwardUnroll = 2;
+
+__host__ __device__ constexpr int half_l(int H, int kk) {
+    constexpr int t[2][kHalfK] = {{1, 2, 3, 4, 1, 2, 3, 4, 1, 2, 3, 4}, {2, 3, 4, 2, 3, 4, 3, 4, 3, 4, 4, 4}};
+    return t[H][kk];
+}
+__host__ __device__ constexpr int half_m(int H, int kk) {
+    return H == 0 ? (kk < 4 ? 0 : 1) : (kk < 6 ? 2 : (kk < 10 ? 3 : 4));
+}
+__host__ __device__ constexpr bool half_sin(int H, int kk) {
+    return H == 0 ? kk >= 8 : kk == 11 || kk == 8 || kk == 9 || (kk >= 3 && kk < 6);
+}
+// N_lm^2 = 2 (l - m)! / (l + m)! (1 for m = 0): the weight of a squared sum of Q_l^m {C_m, S_m},
+// so that g[n][l] = sum_m N_lm^2 (sum_a f_n Q_l^m {C_m, S_m})^2.
+__host__ __device__ constexpr float half_weight(int H, int kk) {
+    const int l = half_l(H, kk), m = half_m(H, kk);
+    if (m == 0) return 1.0f;
+    double num = 2.0, den = 1.0;
+    for (int v = 2; v <= l - m; ++v) num *= v;
+    for (int v = 2; v <= l + m; ++v) den *= v;
+    return (float)(num / den);
+}
+// Q_l^m {C_m, S_m} over the backward's harmonic.
+__host__ __device__ constexpr float half_scale(int H, int kk) {
+    constexpr float t[2][kHalfK] = {{1.0f, 3.0f, 1.5f, 2.5f, 1.0f, 3.0f, 1.5f, 2.5f, 1.0f, 3.0f, 1.5f, 2.5f},
+                                    {3.0f, 15.0f, 7.5f, 3.0f, 15.0f, 7.5f, 15.0f, 105.0f, 15.0f, 105.0f, 105.0f, 105.0f}};
+    return t[H][kk];
 }
 
-// Derivative of f_n with respect to the distance d, together with f_n (same
-// arithmetic as radial_basis_fast for f_n).
-template <int NR>
-__device__ __forceinline__ void radial_basis_grad(float d, float inv_rc, float *f, float *df) {
-    const float u = d * inv_rc, um1 = u - 1.0f;
-    const float x = fmaf(2.0f * um1, um1, -1.0f);
-    float s, c;
-    __sincosf(3.14159265358979f * u, &s, &c);
-    const float hfc = fmaf(0.25f, c, 0.25f);                        // fc / 2
-    const float hdfc = -0.25f * 3.14159265358979f * s * inv_rc;      // (dfc/dd) / 2
-    const float hdxfc = 4.0f * um1 * inv_rc * hfc;                   // (dx/dd) fc / 2
-    float tm1 = 1.0f, t = x, dtm1 = 0.0f, dt = 1.0f;                // T_n and dT_n/dx
-    f[0] = 2.0f * hfc;
-    df[0] = 2.0f * hdfc;
-    if (NR > 1) {
-        f[1] = fmaf(hfc, x, hfc);
-        df[1] = fmaf(hdfc, x, hdfc) + hdxfc;
-    }
-#pragma unroll
-    for (int n = 2; n < NR; ++n) {
-        const float tn = fmaf(2.0f * x, t, -tm1);
-        const float dtn = fmaf(2.0f * x, dt, fmaf(2.0f, t, -dtm1));
-        tm1 = t;
-        t = tn;
-        dtm1 = dt;
-        dt = dtn;
-        f[n] = fmaf(hfc, tn, hfc);
-        df[n] = fmaf(dtn, hdxfc, fmaf(hdfc, tn, hdfc));
-    }
+// Two FP32 multiply-adds in one instruction, each rounded as fmaf.
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+    unsigned long long d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;"
+        : "=l"(d)
+        : "l"(*reinterpret_cast<unsigned long long *>(&a)), "l"(*reinterpret_cast<unsigned long long *>(&b)),
+          "l"(*reinterpret_cast<unsigned long long *>(&c)));
+    return *reinterpret_cast<float2 *>(&d);
+}
+// Element kk of an array of pairs (kk a constant after unrolling).
+__device__ __forceinline__ float &pick(float2 *v, int kk) { return kk & 1 ? v[kk >> 1].y : v[kk >> 1].x; }
+
+// 1 / sqrt(x) to the same two ulp as rsqrtf, without its handling of
+// subnormal arguments (a squared distance is 0 or far above them).
+__device__ __forceinline__ float rsqrt_ftz(float x) {
+    float r;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
 }
 
-// The recurrences behind the harmonics: C_m + i S_m = (x + i y)^m (m <= LMAX)
-// and Q[l][m] = d^m P_l / dz^m (m <= l + 1 <= LMAX + 1; 0 above l).
-template <int LMAX>
-__device__ __forceinline__ void sh_recurrences(float x, float y, float z, float *C, float *S,
-                                               float (&Q)[LMAX + 2][LMAX + 2]) {
+// T_1 .. T_N of x, t[n] = T_n (t[0] unused).
+template <int N>
+__device__ __forceinline__ void chebyshev(float x, float *t) {
+    const float x2 = x + x;
+    t[1] = x;
+    t[2] = fmaf(x2, x, -1.0f);
+#pragma unroll
+    for (int n = 3; n <= N; ++n) t[n] = fmaf(x2, t[n - 1], -t[n - 2]);
+}
+
+// The half's harmonics Q_l^m(z) {C_m, S_m} of the unit vector (x, y, z),
+// Q_l^m = d^m P_l / dz^m by the recurrence in l (what a half does not use is
+// never computed).
+template <int H>
+__device__ __forceinline__ void half_harmonics(float x, float y, float z, float (&Y)[kHalfK]) {
+    constexpr int LM = 4;
+    float C[LM + 1], S[LM + 1], Q[LM + 1][LM + 1];
     C[0] = 1.0f;
     S[0] = 0.0f;
 #pragma unroll
-    for (int m = 1; m <= LMAX; ++m) {
+    for (int m = 1; m <= LM; ++m) {
         C[m] = fmaf(x, C[m - 1], -y * S[m - 1]);
         S[m] = fmaf(x, S[m - 1], y * C[m - 1]);
     }
 #pragma unroll
-    for (int l = 0; l <= LMAX + 1; ++l)
+    for (int m = 0; m <= LM; ++m) {
 #pragma unroll
-        for (int m = 0; m <= LMAX + 1; ++m) Q[l][m] = 0.0f;
-#pragma unroll
-    for (int m = 0; m <= LMAX; ++m) {
-#pragma unroll
-        for (int l = m; l <= LMAX; ++l) {
+        for (int l = m; l <= LM; ++l) {
             if (l == m) Q[l][m] = (float)dfact_odd(m);
             else if (l == m + 1) Q[l][m] = (float)(2 * m + 1) * z * Q[l - 1][m];
             else
@@ -164,104 +207,86 @@ __device__ __forceinline__ void sh_recurrences(float x, float y, float z, float 
                           (1.0f / (float)(l - m));
         }
     }
-}
-
-__host__ __device__ constexpr int sh_m_of(int k) {  // m of harmonic index k (order m = 0, (cos, sin) m = 1..l)
-    return (k + 1 - sh_l_of(k) * sh_l_of(k) + 1) / 2;
-}
-__host__ __device__ constexpr bool sh_is_sin(int k) {
-    return sh_m_of(k) > 0 && ((k + 1 - sh_l_of(k) * sh_l_of(k)) % 2 == 0);
-}
-
-// Weight of harmonic k in the angular descriptor when the harmonics are kept
-// unnormalised (Q_l^m {C_m, S_m}): N_lm^2 = 2 (l-m)! / (l+m)! for m >= 1, 1 for
-// m = 0, so that g[n][l] = sum_m N_lm^2 (sum_a f_n Q_l^m {C_m, S_m})^2.
-__host__ __device__ constexpr float sh_weight(int k) {
-    const int l = sh_l_of(k), m = sh_m_of(k);
-    if (m == 0) return 1.0f;
-    double num = 2.0, den = 1.0;
-    for (int v = 2; v <= l - m; ++v) num *= v;
-    for (int v = 2; v <= l + m; ++v) den *= v;
-    return (float)(num / den);
-}
-
-// The unnormalised harmonics Q_l^m {C_m, S_m} (m > 0) and Q_l^0 of this half
-// (indices k0 .. k0 + KC - 1, zero past K) from the recurrences.
-template <class Cfg, int KC, int k0>
-__device__ __forceinline__ void sh_half_u(const float *C, const float *Sn,
-                                          const float (&Q)[Cfg::LMAX + 2][Cfg::LMAX + 2], float *Y) {
 #pragma unroll
-    for (int kk = 0; kk < KC; ++kk) {
-        const int k = k0 + kk;
-        if (k < Cfg::K) {
-            const int l = sh_l_of(k), m = sh_m_of(k);
-            Y[kk] = m == 0 ? Q[l][0] : Q[l][m] * (sh_is_sin(k) ? Sn[m] : C[m]);
-        } else {
-            Y[kk] = 0.f;
-        }
+    for (int kk = 0; kk < kHalfK; ++kk) {
+        const int l = half_l(H, kk), m = half_m(H, kk);
+        Y[kk] = m == 0 ? Q[l][0] : Q[l][m] * (half_sin(H, kk) ? S[m] : C[m]);
     }
 }
 
+// s plus the weighted squares of row n's sums over the half's harmonics k0 .. k1 - 1 of degree l.
+template <int H>
+__device__ __forceinline__ float add_squares(float2 *An, int l, int k0, int k1, float s) {
+#pragma unroll
+    for (int kk = 0; kk < kHalfK; ++kk)
+        if (kk >= k0 && kk < k1 && half_l(H, kk) == l) s = fmaf(half_weight(H, kk) * pick(An, kk), pick(An, kk), s);
+    return s;
+}
+
+// Forward of one half: A[n][k] = sum_a f_n(a) Y_k(a), kept in the caller's
+// registers for the backward, and its share of the descriptor row gp[0..47]: half
+// 0 the radial sums n = 0..5 and, per (n, l), its weighted squares; half 1 the
+// radial sums n = 6..10 and the padding column. half_forward_finish adds half 1's
+// squares. r holds the pair's 2 npts centred points (x, y, z each).
+template <class Cfg, int H, int UNROLL>
+__device__ __forceinline__ void half_forward(const float *r, int npts, float inv_rc, float *gp,
+                                              float2 (&A)[Cfg::NA][kHalfP]) {
+    static_assert(Cfg::LMAX == 4 && Cfg::K == 2 * kHalfK && Cfg::NA == 9 && Cfg::NR == 11, "hypers (10, 8, 4)");
+    constexpr int NR = Cfg::NR, NA = Cfg::NA, NS = 6;  // radial sums split at n = NS
+    constexpr int NT = H == 0 ? NA - 1 : NR - 1;       // Chebyshev polynomials this half needs
+#pragma unroll
+    for (int n = 0; n < NA; ++n)
+#pragma unroll
+        for (int k2 = 0; k2 < kHalfP; ++k2) A[n][k2] = make_float2(0.f, 0.f);
+    float R[NR];
+#pragma unroll
+    for (int n = 0; n < NR; ++n) R[n] = 0.f;
+#pragma unroll UNROLL
+    for (int a = 2 * npts; a > 0; --a, r += 3) {
+        const float rx = r[0], ry = r[1], rz = r[2];
+        const float d2 = fmaf(rx, rx, fmaf(ry, ry, rz * rz));
+        const float inv_d = rsqrt_ftz(d2);
+        const float u = d2 * inv_d * inv_rc, um1 = u - 1.0f;
+        // the hardware cosine (an absolute error of a few 1e-7 for the arguments here, far
+        // below the tensor-core net's 1e-5)
+        const float h = fmaf(0.25f, __cosf(3.14159265358979f * u), 0.25f);  // fc / 2
+        float f[NT + 1], Y[kHalfK];
+        chebyshev<NT>(fmaf(2.0f * um1, um1, -1.0f), f);
+        half_harmonics<H>(rx * inv_d, ry * inv_d, rz * inv_d, Y);
+#pragma unroll
+        for (int n = 0; n <= NT; ++n) f[n] = n == 0 ? 2.0f * h : fmaf(h, f[n], h);
+#pragma unroll
+        for (int n = H == 0 ? 0 : NS; n < (H == 0 ? NS : NR); ++n) R[n] += f[n];
+#pragma unroll
+        for (int n = 0; n < NA; ++n)
+#pragma unroll
+            for (int k2 = 0; k2 < kHalfP; ++k2)
+                A[n][k2] = fma2(make_float2(f[n], f[n]), make_float2(Y[2 * k2], Y[2 * k2 + 1]), A[n][k2]);
+    }
+#pragma unroll
+    for (int n = H == 0 ? 0 : NS; n < (H == 0 ? NS : NR); ++n) gp[n] = R[n];
+    if (H == 1) {
+        gp[Cfg::D] = 0.f;
+        return;
+    }
+#pragma unroll
+    for (int n = 0; n < NA; ++n)
+#pragma unroll
+        for (int l = 1; l <= Cfg::LMAX; ++l) gp[NR + n * Cfg::LMAX + l - 1] = add_squares<H>(A[n], l, 0, kHalfK, 0.f);
+}
+
+// Half 1's weighted squares onto half 0's in the row gp (after a barrier). The
+// squares of one (n, l) add up in the order of the index split, l = 1, 2 and the
+// first four of l = 3 before the rest: the descriptor stays the same to the bit,
+// and with it the branch a ReLU net takes and the slope of a saturated unit.
 template <class Cfg>
-struct Half {
-    static constexpr int KC = (Cfg::K + 1) / 2;  // harmonics per half
-};
-
-// sum_a f_n(a) Y_k(a) for this half's harmonics k0..k0+KC-1, unnormalised (and
-// the radial sums). r holds the pair's nd centred points (x, y, z each).
-template <class Cfg, int KC, int k0>
-__device__ __forceinline__ void accumulate_A(const float *r, int nd, float inv_rc, float (*A)[KC], float *R) {
+__device__ __forceinline__ void half_forward_finish(float *gp, float2 (&A)[Cfg::NA][kHalfP]) {
 #pragma unroll
-    for (int n = 0; n < Cfg::NA; ++n)
-#pragma unroll
-        for (int kk = 0; kk < KC; ++kk) A[n][kk] = 0.f;
-#pragma unroll
-    for (int n = 0; n < Cfg::NR; ++n) R[n] = 0.f;
-    for (int a = 0; a < nd; ++a) {
-        const float rx = r[3 * a], ry = r[3 * a + 1], rz = r[3 * a + 2];
-        float d2 = fmaf(rx, rx, fmaf(ry, ry, rz * rz));
-        float inv_d = rsqrtf(d2);
-        float f[Cfg::NR];
-        radial_basis_fast<Cfg::NR>(d2 * inv_d, inv_rc, f);
-#pragma unroll
-        for (int n = 0; n < Cfg::NR; ++n) R[n] += f[n];
-        constexpr int LM = Cfg::LMAX;
-        float C[LM + 1], Sn[LM + 1], Q[LM + 2][LM + 2];
-        sh_recurrences<LM>(rx * inv_d, ry * inv_d, rz * inv_d, C, Sn, Q);
-        float Y[KC];
-        sh_half_u<Cfg, KC, k0>(C, Sn, Q, Y);
-#pragma unroll
-        for (int n = 0; n < Cfg::NA; ++n)
-#pragma unroll
-            for (int kk = 0; kk < KC; ++kk)
-                if (k0 + kk < Cfg::K) A[n][kk] = fmaf(f[n], Y[kk], A[n][kk]);
-    }
-}
-
-// Forward of one half of the harmonics: radial sums (half 0) and the partial
-// sums of weighted squares of this half's harmonics, written to gp[0..47]
-// (zeros elsewhere). The unnormalised sums A of this half stay in the caller's
-// registers for the backward.
-template <class Cfg, int H>
-__device__ __forceinline__ void half_forward(const float *r, int nd, float inv_rc, float *gp,
-                                             float (&A)[Cfg::NA][Half<Cfg>::KC]) {
-    constexpr int KC = Half<Cfg>::KC;
-    float Rr[Cfg::NR];
-    accumulate_A<Cfg, KC, H * KC>(r, nd, inv_rc, A, Rr);
-    for (int k = 0; k < 48; ++k) gp[k] = 0.f;
-    if (H == 0) {
-#pragma unroll
-        for (int n = 0; n < Cfg::NR; ++n) gp[n] = Rr[n];
-    }
-#pragma unroll
-    for (int kk = 0; kk < KC; ++kk) {
-        if (H * KC + kk < Cfg::K) {
-            const int l = sh_l_of(H * KC + kk);
-            const float w = sh_weight(H * KC + kk);
-#pragma unroll
-            for (int n = 0; n < Cfg::NA; ++n)
-                gp[Cfg::NR + n * Cfg::LMAX + l - 1] = fmaf(w * A[n][kk], A[n][kk], gp[Cfg::NR + n * Cfg::LMAX + l - 1]);
-        }
+    for (int n = 0; n < Cfg::NA; ++n) {
+        float *g = gp + Cfg::NR + n * Cfg::LMAX;
+        g[1] = add_squares<1>(A[n], 2, 0, kHalfK, g[1]);
+        g[2] = add_squares<1>(A[n], 3, 0, 3, g[2]) + add_squares<1>(A[n], 3, 3, kHalfK, 0.f);
+        g[3] = add_squares<1>(A[n], 4, 0, kHalfK, g[3]);
     }
 }
 
@@ -269,131 +294,197 @@ __device__ __forceinline__ void half_forward(const float *r, int nd, float inv_r
 // (overwritten), the partial sums over the centred points r_a of dE/dr_a
 // needed for the pair force and torques: sum_{a in i} G_a, sum_a G_a,
 // sum_{a in i} r_a x G_a, sum_{a in j} r_a x G_a -> out[12] (the caller adds
-// the centroid terms).
+// the centroid terms). Per point, with G_nk = dE/dA_nk,
+//   phi = h sum_k q_k Y_k + h p  (p: the radial descriptor's polynomial, half 0),
+//   dphi/dd = h' (sum_k q_k Y_k + p) + h x' (sum_n s_n T_n'(x)),  s_n = sum_k G_nk Y_k (+ dE/dg_n),
+// the last sum by Clenshaw's recurrence on T_n' = n U_(n-1). The angular
+// gradient is h sum_k q_k grad Y_k, assembled from the sums U, V (over the
+// half's cos and sin harmonics of one order m, times their polynomial in z)
+// and W, X (the same with its derivative):
+//   gx = sum_m m (U C_(m-1) + V S_(m-1)), gy = sum_m m (V C_(m-1) - U S_(m-1)),
+//   gz = sum_m W C_m + X S_m, sum_k q_k Y_k = sum_m U C_m + V S_m (m >= 1) and
+//   x gx + y gy = sum_m m (U C_m + V S_m).
 template <class Cfg, int H>
 __device__ __forceinline__ void half_backward(const float *r, int npts, float inv_rc, const float *dg, float *out,
-                                              float (&A)[Cfg::NA][Half<Cfg>::KC]) {
-    constexpr int KC = Half<Cfg>::KC;
+                                               float2 (&A)[Cfg::NA][kHalfP]) {
+    constexpr int NR = Cfg::NR, NA = Cfg::NA;
+    constexpr int NT = H == 0 ? NR - 1 : NA - 1;
 #pragma unroll
-    for (int kk = 0; kk < KC; ++kk) {
-        if (H * KC + kk < Cfg::K) {
-            const int l = sh_l_of(H * KC + kk);
-            const float w2 = 2.0f * sh_weight(H * KC + kk);
+    for (int kk = 0; kk < kHalfK; ++kk) {
+        const float w2 = 2.0f * half_weight(H, kk) * half_scale(H, kk);
+        float s = 0.f;
 #pragma unroll
-            for (int n = 0; n < Cfg::NA; ++n) A[n][kk] *= w2 * dg[Cfg::NR + n * Cfg::LMAX + l - 1];
+        for (int n = 0; n < NA; ++n) {
+            float &a = pick(A[n], kk);
+            a *= w2 * dg[NR + n * Cfg::LMAX + half_l(H, kk) - 1];
+            s += a;
+        }
+        pick(A[0], kk) += s;  // coefficient of 1: sum_n G_nk, and T_0 = 1 once more for n = 0
+    }
+    float gr[NR];  // the same of the radial descriptor
+    if (H == 0) {
+        float s = 0.f;
+#pragma unroll
+        for (int n = 0; n < NR; ++n) {
+            gr[n] = dg[n];
+            s += gr[n];
+        }
+        gr[0] += s;
+    }
+    float Si[3], Xi[3];
+#pragma unroll 1  // the same code for both bodies: one set of sums, no branch per point
+    for (int body = 0; body < 2; ++body) {
+        float G[3] = {0, 0, 0}, X[3] = {0, 0, 0};
+#pragma unroll kBackwardUnroll
+        for (int a = npts; a > 0; --a, r += 3) {
+            const float rx = r[0], ry = r[1], rz = r[2];
+            const float d2 = fmaf(rx, rx, fmaf(ry, ry, rz * rz));
+            const float inv_d = rsqrt_ftz(d2);
+            const float x = rx * inv_d, y = ry * inv_d, z = rz * inv_d, z2 = z * z;
+            const float u = d2 * inv_d * inv_rc, um1 = u - 1.0f;
+            float sn, cs;
+            __sincosf(3.14159265358979f * u, &sn, &cs);
+            const float h = fmaf(0.25f, cs, 0.25f);                        // fc / 2
+            const float hd = (-0.25f * 3.14159265358979f * inv_rc) * sn;    // dh/dd
+            const float hdx = (4.0f * inv_rc) * um1 * h;                    // h dx/dd
+            const float cx = fmaf(2.0f * um1, um1, -1.0f), cx2 = cx + cx;
+            float t[NT + 1], Y[kHalfK], q[kHalfK], s[NA];
+            chebyshev<NT>(cx, t);
+            // the harmonics, and the polynomials and powers that the gradient needs too
+            float c3 = 0.f, c4 = 0.f, c7 = 0.f;
+            if (H == 0) {
+                c3 = fmaf(5.0f, z2, -1.0f), c4 = z * fmaf(7.0f, z2, -3.0f);
+                Y[0] = z;
+                Y[1] = fmaf(0.5f, z2, -1.0f / 6.0f);
+                Y[2] = z * fmaf(5.0f / 3.0f, z2, -1.0f);
+                Y[3] = fmaf(z2, fmaf(1.75f, z2, -1.5f), 0.15f);
+                Y[4] = x, Y[5] = x * z, Y[6] = x * c3, Y[7] = x * c4;
+                Y[8] = y, Y[9] = y * z, Y[10] = y * c3, Y[11] = y * c4;
+            } else {
+                c7 = fmaf(7.0f, z2, -1.0f);
+                const float C2 = fmaf(x, x, -y * y), S2 = (x + x) * y;
+                const float C3 = fmaf(x, C2, -y * S2), S3 = fmaf(x, S2, y * C2);
+                Y[0] = C2, Y[1] = C2 * z, Y[2] = C2 * c7;
+                Y[3] = S2, Y[4] = S2 * z, Y[5] = S2 * c7;
+                Y[6] = C3, Y[7] = C3 * z, Y[8] = S3, Y[9] = S3 * z;
+                Y[10] = fmaf(C2, C2, -S2 * S2), Y[11] = (C2 + C2) * S2;
+            }
+#pragma unroll
+            for (int k2 = 0; k2 < kHalfP; ++k2) {
+                float2 v = A[0][k2];
+#pragma unroll
+                for (int n = 1; n < NA; ++n) v = fma2(A[n][k2], make_float2(t[n], t[n]), v);
+                q[2 * k2] = v.x;
+                q[2 * k2 + 1] = v.y;
+            }
+#pragma unroll
+            for (int n = 1; n < NA; ++n) {
+                float2 v = make_float2(H == 0 ? gr[n] : 0.f, 0.f);
+#pragma unroll
+                for (int k2 = 0; k2 < kHalfP; ++k2) v = fma2(A[n][k2], make_float2(Y[2 * k2], Y[2 * k2 + 1]), v);
+                s[n] = v.x + v.y;
+            }
+            // sum_n s_n n U_(n-1)(cx), n descending
+            float b1 = 0.f, b2 = 0.f;
+            if (H == 0) {
+                b2 = (float)(NR - 1) * gr[NR - 1];
+                b1 = fmaf(cx2, b2, (float)(NR - 2) * gr[NR - 2]);
+            }
+#pragma unroll
+            for (int n = NA - 1; n >= 1; --n) {
+                const float b0 = fmaf(cx2, b1, fmaf((float)n, s[n], -b2));
+                b2 = b1;
+                b1 = b0;
+            }
+            float gx, gy, gz, e, phi;  // sum_k q_k grad Y_k, x gx + y gy, sum_k q_k Y_k (+ the radial polynomial)
+            if (H == 0) {
+                const float z10 = 10.0f * z, c21 = fmaf(21.0f, z2, -3.0f);
+                gx = fmaf(q[7], c4, fmaf(q[6], c3, fmaf(q[5], z, q[4])));
+                gy = fmaf(q[11], c4, fmaf(q[10], c3, fmaf(q[9], z, q[8])));
+                const float W0 = fmaf(q[3], c4, fmaf(q[2], c3, fmaf(q[1], z, q[0])));
+                const float W1 = fmaf(q[7], c21, fmaf(q[6], z10, q[5])), X1 = fmaf(q[11], c21, fmaf(q[10], z10, q[9]));
+                gz = fmaf(x, W1, fmaf(y, X1, W0));
+                e = fmaf(x, gx, y * gy);
+                float p = gr[0];
+#pragma unroll
+                for (int n = 1; n < NR; ++n) p = fmaf(gr[n], t[n], p);
+                phi = fmaf(q[0], Y[0], fmaf(q[1], Y[1], fmaf(q[2], Y[2], fmaf(q[3], Y[3], e)))) + p;
+            } else {
+                const float z14 = 14.0f * z, C2 = Y[0], S2 = Y[3], C3 = Y[6], S3 = Y[8];
+                const float U2 = fmaf(q[2], c7, fmaf(q[1], z, q[0])), V2 = fmaf(q[5], c7, fmaf(q[4], z, q[3]));
+                const float U3 = fmaf(q[7], z, q[6]), V3 = fmaf(q[9], z, q[8]);
+                const float W2 = fmaf(q[2], z14, q[1]), X2 = fmaf(q[5], z14, q[4]);
+                const float x2 = x + x, y2 = y + y, C23 = 3.0f * C2, S23 = 3.0f * S2, C34 = 4.0f * C3, S34 = 4.0f * S3;
+                gx = fmaf(U2, x2, fmaf(V2, y2, fmaf(U3, C23, fmaf(V3, S23, fmaf(q[10], C34, q[11] * S34)))));
+                gy = fmaf(V2, x2, fmaf(-U2, y2, fmaf(V3, C23, fmaf(-U3, S23, fmaf(q[11], C34, -q[10] * S34)))));
+                gz = fmaf(W2, C2, fmaf(X2, S2, fmaf(q[7], C3, q[9] * S3)));
+                const float w2 = fmaf(U2, C2, V2 * S2), w3 = fmaf(U3, C3, V3 * S3), w4 = fmaf(q[10], Y[10], q[11] * Y[11]);
+                e = fmaf(4.0f, w4, fmaf(3.0f, w3, w2 + w2));
+                phi = w2 + w3 + w4;
+            }
+            // dE/dr = phi' rhat + (h g - rhat (rhat . h g)) / d
+            const float hi = h * inv_d;
+            const float dot = fmaf(z, gz, e);
+            const float c1 = fmaf(-dot, hi, fmaf(hd, phi, hdx * b1));
+            const float Gx = fmaf(x, c1, gx * hi);
+            const float Gy = fmaf(y, c1, gy * hi);
+            const float Gz = fmaf(z, c1, gz * hi);
+            G[0] += Gx;
+            G[1] += Gy;
+            G[2] += Gz;
+            X[0] += ry * Gz - rz * Gy;
+            X[1] += rz * Gx - rx * Gz;
+            X[2] += rx * Gy - ry * Gx;
+        }
+        if (body == 0) {
+#pragma unroll
+            for (int k = 0; k < 3; ++k) Si[k] = G[k], Xi[k] = X[k];
         } else {
 #pragma unroll
-            for (int n = 0; n < Cfg::NA; ++n) A[n][kk] = 0.f;
-        }
-    }
-    float grad_rad[Cfg::NR];
-#pragma unroll
-    for (int n = 0; n < Cfg::NR; ++n) grad_rad[n] = H == 0 ? dg[n] : 0.f;
-    float Si[3] = {0, 0, 0}, Sj[3] = {0, 0, 0}, Xi[3] = {0, 0, 0}, Xj[3] = {0, 0, 0};
-    const int nd = 2 * npts;
-    for (int a = 0; a < nd; ++a) {
-        const float rx = r[3 * a], ry = r[3 * a + 1], rz = r[3 * a + 2];
-        float d2 = fmaf(rx, rx, fmaf(ry, ry, rz * rz));
-        float inv_d = rsqrtf(d2);
-        float d = d2 * inv_d;
-        float ux = rx * inv_d, uy = ry * inv_d, uz = rz * inv_d;
-        float f[Cfg::NR], df[Cfg::NR];
-        radial_basis_grad<Cfg::NR>(d, inv_rc, f, df);
-        constexpr int LM = Cfg::LMAX;
-        float C[LM + 1], Sn[LM + 1], Q[LM + 2][LM + 2];
-        sh_recurrences<LM>(ux, uy, uz, C, Sn, Q);
-        float Y[KC];
-        sh_half_u<Cfg, KC, H * KC>(C, Sn, Q, Y);
-        float gr = 0.f;
-#pragma unroll
-        for (int n = 0; n < Cfg::NR; ++n) {
-            float s = grad_rad[n];
-            if (n < Cfg::NA) {
-#pragma unroll
-                for (int kk = 0; kk < KC; ++kk)
-                    if (H * KC + kk < Cfg::K) s = fmaf(A[n][kk], Y[kk], s);
-            }
-            gr = fmaf(s, df[n], gr);
-        }
-        // gradient of sum_k s_k Y_k grouped by m: with U_m, V_m the sums of
-        // s m Q_l^m over the cos / sin harmonics of order m and Wc_m, Ws_m those
-        // of s Q_l^(m+1),
-        //   gx = sum_m U_m C_(m-1) + V_m S_(m-1), gy = sum_m V_m C_(m-1) - U_m S_(m-1),
-        //   gz = sum_m Wc_m C_m + Ws_m S_m.
-        float U[LM + 1], V[LM + 1], Wc[LM + 1], Ws[LM + 1];
-#pragma unroll
-        for (int m = 0; m <= LM; ++m) U[m] = V[m] = Wc[m] = Ws[m] = 0.f;
-#pragma unroll
-        for (int kk = 0; kk < KC; ++kk) {
-            const int k = H * KC + kk;
-            if (k < Cfg::K) {
-                float s = 0.f;
-#pragma unroll
-                for (int n = 0; n < Cfg::NA; ++n) s = fmaf(A[n][kk], f[n], s);
-                const int l = sh_l_of(k), m = sh_m_of(k);
-                if (sh_is_sin(k)) {
-                    V[m] = fmaf(s, m == 1 ? Q[l][m] : (float)m * Q[l][m], V[m]);
-                    Ws[m] = fmaf(s, Q[l][m + 1], Ws[m]);
-                } else {
-                    if (m > 0) U[m] = fmaf(s, m == 1 ? Q[l][m] : (float)m * Q[l][m], U[m]);
-                    Wc[m] = fmaf(s, Q[l][m + 1], Wc[m]);
-                }
+            for (int k = 0; k < 3; ++k) {
+                out[k] = Si[k];
+                out[3 + k] = Si[k] + G[k];
+                out[6 + k] = Xi[k];
+                out[9 + k] = X[k];
             }
         }
-        float gx = 0.f, gy = 0.f, gz = Wc[0];
-#pragma unroll
-        for (int m = 1; m <= LM; ++m) {
-            gx = fmaf(U[m], C[m - 1], fmaf(V[m], Sn[m - 1], gx));
-            gy = fmaf(V[m], C[m - 1], fmaf(-U[m], Sn[m - 1], gy));
-            gz = fmaf(Wc[m], C[m], fmaf(Ws[m], Sn[m], gz));
-        }
-        // dE/dr = gr rhat + (g - rhat (rhat . g)) / d = rhat (gr - (rhat . g) / d) + g / d
-        const float dot = ux * gx + uy * gy + uz * gz;
-        const float c1 = fmaf(-dot, inv_d, gr);
-        const float Gx = fmaf(ux, c1, gx * inv_d);
-        const float Gy = fmaf(uy, c1, gy * inv_d);
-        const float Gz = fmaf(uz, c1, gz * inv_d);
-        if (a < npts) {
-            Si[0] += Gx;
-            Si[1] += Gy;
-            Si[2] += Gz;
-            Xi[0] += ry * Gz - rz * Gy;
-            Xi[1] += rz * Gx - rx * Gz;
-            Xi[2] += rx * Gy - ry * Gx;
-        } else {
-            Sj[0] += Gx;
-            Sj[1] += Gy;
-            Sj[2] += Gz;
-            Xj[0] += ry * Gz - rz * Gy;
-            Xj[1] += rz * Gx - rx * Gz;
-            Xj[2] += rx * Gy - ry * Gx;
-        }
-    }
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-        out[k] = Si[k];
-        out[3 + k] = Si[k] + Sj[k];
-        out[6 + k] = Xi[k];
-        out[9 + k] = Xj[k];
     }
 }
 
 struct AdjShared {
-    float *R;          // rotated body points, kAP x rs (aliases the MLP operand area)
+    float *R;          // rotated body points, NP x rs (may alias the MLP operand area)
     char *ops;         // MLP operand area (bf16 hi/lo tiles)
     char *wts;         // weights (bf16 hi/lo), resident
     float *par;        // biases + last-layer weights (fp32)
-    float *g0, *g1;    // per-half descriptor partials, kAP x kGS each; g0 later holds dE/dg
-    float *t;          // translations, kAP x 3
-    float *cen;        // centroids, kAP x 3
-    float *part;       // per-half gradient partial sums, 2 x kAP x kPartStride
-    float *eps;        // per-half energy partials, 2 x kAP
-    float *fd;         // per-pair F, T_i, T_j, kAP x 9
-    int *ij;           // pair indices, kAP x 2
+    float *g;          // descriptor rows, then dE/dg, NP x kGS
+    float *t;          // translations, NP x 3
+    float *cen;        // centroids, NP x 3
+    float *part;       // per-half gradient partial sums, 2 x NP x kPartStride
+    float *eps;        // per-half energy partials, 2 x NP
+    float *fd;         // per-pair F, T_i, T_j, NP x 9
+    int *ij;           // pair indices, NP x 2
     float *pts;        // body points
-    float4 *q;         // orientations of the tile's pairs, kAP x 2 (i, j)
+    float4 *q;         // orientations of the tile's pairs, NP x 2 (i, j)
     float *psum;       // sum of the body points (body frame), 3
 };
+
+// Per-pair areas of a tile of NP pairs (the fused kernel's and the wide path's
+// descriptor kernels'), taken from `base`.
+template <int NP>
+constexpr size_t pair_area_bytes() {
+    return (size_t)NP * 4 * (8 + 3 + 3 + 2 + 2 + 2 * kPartStride + 9);
+}
+template <int NP>
+__device__ __forceinline__ void take_pair_areas(AdjShared &S, char *base) {
+    float *f = reinterpret_cast<float *>(base);
+    S.q = reinterpret_cast<float4 *>(f);
+    S.t = f + 8 * NP;
+    S.cen = f + 11 * NP;
+    S.eps = f + 14 * NP;
+    S.ij = reinterpret_cast<int *>(f + 16 * NP);
+    S.part = f + 18 * NP;
+    S.fd = S.part + 2 * NP * kPartStride;
+}
 
 // Sum of the body-frame points into S.psum (one warp; call before a barrier).
 __device__ __forceinline__ void body_point_sum(const AdjShared &S, int npts) {
@@ -485,13 +576,13 @@ __device__ __forceinline__ void store_centroid(const AdjShared &S, int q, int np
 
 // Centred cloud points of the tile's pairs into S.R: row q holds body i's
 // points R_i b_a - c, then body j's R_j b_a + t - c (c = S.cen). Thread
-// (q, body) = (tid % kAP, tid / kAP) rotates all points of one body of one pair
+// (q, body) = (tid % NP, tid / NP) rotates all points of one body of one pair
 // (body points broadcast from shared memory, rows of odd stride rs: no bank
 // conflicts, no index divisions) with the matrix of q v q* for q = (w, u),
 // (w^2 - |u|^2) I + 2 u u^T + 2 w [u]x, built once: 9 FMAs per point.
+template <int NP>
 __device__ __forceinline__ void rotate_tile(const AdjShared &S, int npts, int rs) {
-    static_assert(kAThreads == 2 * kAP, "one thread per (pair, body)");
-    const int q = threadIdx.x & (kAP - 1), body = threadIdx.x / kAP;
+    const int q = threadIdx.x & (NP - 1), body = threadIdx.x / NP;
     const float4 qq = S.q[2 * q + body];
     const float w = qq.x, x = qq.y, y = qq.z, z = qq.w;
     const float a0 = w * w - (x * x + y * y + z * z);
@@ -526,6 +617,131 @@ __device__ __forceinline__ void add_centroid_terms(const AdjShared &S, int q, co
     Xj[2] += e[0] * Sj[1] - e[1] * Sj[0];
 }
 
+// Pair indices, orientations, translations and centroids of the tile's pairs
+// p0 .. p0 + NP - 1 (past the last pair: that pair again), then their rotated,
+// centred points into S.R.
+template <int NP, bool MULTI>
+__device__ __forceinline__ void load_pairs(const AdjShared &S, const float *pos, const float *quat, float L,
+                                           const int *pairs, long long P, long long p0, int npts, int rs,
+                                           const int *rep, const amlp_replica *rp) {
+    const int tid = threadIdx.x;
+    if (tid < NP) {
+        long long pr = min(p0 + tid, P - 1);
+        int i = pairs[2 * pr], j = pairs[2 * pr + 1];
+        S.q[2 * tid] = load_quat(quat, i);
+        S.q[2 * tid + 1] = load_quat(quat, j);
+        float dd;
+        float3 tt = min_image(pos, i, j, MULTI ? rp[rep[i]].box : L, &dd);
+        S.t[3 * tid] = tt.x;
+        S.t[3 * tid + 1] = tt.y;
+        S.t[3 * tid + 2] = tt.z;
+        S.ij[2 * tid] = i;
+        S.ij[2 * tid + 1] = j;
+        store_centroid(S, tid, npts);
+    }
+    __syncthreads();
+    rotate_tile<NP>(S, npts, rs);
+}
+
+// Per-pair force/torque from the two halves' partial sums, scaled, clipped
+// (unless clip == 0), then scattered with runs of equal i summed in the warp
+// (the first NP threads, thread = pair). y_of(q) is the net output of the tile's pair q.
+template <int NP, bool MULTI, class Y>
+__device__ __forceinline__ void adj_finish_tile(const AdjShared &S, int npts, int valid, float en_min, float en_range,
+                                                const Y &y_of, float *F, float *T, double *pe, const int *rep,
+                                                double &pe_acc, int clip) {
+    const int tid = threadIdx.x, lane = tid & 31;
+    const int nd = 2 * npts;
+    if (tid < NP) {
+        const int p = tid;
+        const float *a0 = S.part + p * kPartStride, *a1 = a0 + NP * kPartStride;
+        float Si[3], Sa[3], Xi[3], Xj[3];
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            Si[k] = a0[k] + a1[k];
+            Sa[k] = a0[3 + k] + a1[3 + k];
+            Xi[k] = a0[6 + k] + a1[6 + k];
+            Xj[k] = a0[9 + k] + a1[9 + k];
+        }
+        add_centroid_terms(S, p, Si, Sa, Xi, Xj);
+        const float3 ps = make_float3(S.psum[0], S.psum[1], S.psum[2]);
+        const float3 pi3 = rotate_ref(S.q[2 * p], ps), qj3 = rotate_ref(S.q[2 * p + 1], ps);
+        const float Pi[3] = {pi3.x, pi3.y, pi3.z}, Qj[3] = {qj3.x, qj3.y, qj3.z};
+        const float inv_nd = 1.0f / (float)nd;
+        float Gm[3] = {Sa[0] * inv_nd, Sa[1] * inv_nd, Sa[2] * inv_nd};
+        float Fp[3], Ti[3], Tj[3];
+#pragma unroll
+        for (int k = 0; k < 3; ++k) Fp[k] = -(Si[k] - (float)npts * Gm[k]);
+        Ti[0] = -(Xi[0] - (Pi[1] * Gm[2] - Pi[2] * Gm[1]));
+        Ti[1] = -(Xi[1] - (Pi[2] * Gm[0] - Pi[0] * Gm[2]));
+        Ti[2] = -(Xi[2] - (Pi[0] * Gm[1] - Pi[1] * Gm[0]));
+        Tj[0] = -(Xj[0] - (Qj[1] * Gm[2] - Qj[2] * Gm[1]));
+        Tj[1] = -(Xj[1] - (Qj[2] * Gm[0] - Qj[0] * Gm[2]));
+        Tj[2] = -(Xj[2] - (Qj[0] * Gm[1] - Qj[1] * Gm[0]));
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            float f = Fp[k] * en_range, ti = Ti[k] * en_range, tj = Tj[k] * en_range;
+            S.fd[9 * p + k] = clip ? clip100(f) : f;
+            S.fd[9 * p + 3 + k] = clip ? clip100(ti) : ti;
+            S.fd[9 * p + 6 + k] = clip ? clip100(tj) : tj;
+        }
+        if (!MULTI && p < valid) pe_acc += (double)en_min + (double)en_range * (double)y_of(p);
+    }
+    __syncthreads();
+    if (tid < NP) {
+        const int q = tid;
+        const bool ok = q < valid;
+        const int i = S.ij[2 * q], j = S.ij[2 * q + 1];
+        float v[6];
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            v[k] = ok ? S.fd[9 * q + k] : 0.f;
+            v[3 + k] = ok ? S.fd[9 * q + 3 + k] : 0.f;
+        }
+        if (ok) {
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+                atomicAdd(F + 3 * j + k, -v[k]);
+                atomicAdd(T + 3 * j + k, S.fd[9 * q + 6 + k]);
+            }
+        }
+        const bool runs = warp_keys_sorted(i, ok);  // every lane takes part (warp vote)
+        int key = ok && runs ? i : -1 - q;  // unsorted pairs: no merging
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            int ko = __shfl_up_sync(0xffffffffu, key, o);
+#pragma unroll
+            for (int k = 0; k < 6; ++k) {
+                float yv = __shfl_up_sync(0xffffffffu, v[k], o);
+                if (lane >= o && ko == key) v[k] += yv;
+            }
+        }
+        int kn = __shfl_down_sync(0xffffffffu, key, 1);
+        if (ok && (lane == 31 || kn != key)) {
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+                atomicAdd(F + 3 * i + k, v[k]);
+                atomicAdd(T + 3 * i + k, v[3 + k]);
+            }
+        }
+        if (MULTI && pe) {
+            double e = ok ? (double)en_min + (double)en_range * (double)y_of(q) : 0.0;
+            const int sys = ok ? rep[i] : 0;
+            const bool sys_runs = warp_keys_sorted(sys, ok);
+            int rk = ok && sys_runs ? sys : -1 - lane;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                int ro = __shfl_up_sync(0xffffffffu, rk, o);
+                double yv = __shfl_up_sync(0xffffffffu, e, o);
+                if (lane >= o && ro == rk) e += yv;
+            }
+            int rn = __shfl_down_sync(0xffffffffu, rk, 1);
+            if (ok && (lane == 31 || rn != rk)) atomicAdd(pe + sys, e);
+        }
+    }
+    __syncthreads();
+}
+
 // MULTI: the pairs come from many systems in one launch; body i's system is
 // rep[i], its box rp[rep[i]].box, and the pair energies are summed per system
 // into pe[rep[i]].
@@ -536,7 +752,6 @@ __global__ void __launch_bounds__(kAThreads, 1) k_forces_adjoint(const float *po
                                                                 float en_range, AdjNet net, const float *w, float *F,
                                                                 float *T, double *pe, const int *rep,
                                                                 const amlp_replica *rp, int keep_r) {
-    constexpr int KC = Half<Cfg>::KC;
     constexpr int DP = kGS;  // row stride of the fp32 descriptor staging
     extern __shared__ __align__(128) char smem_raw[];
     __shared__ uint64_t mbar;
@@ -544,7 +759,7 @@ __global__ void __launch_bounds__(kAThreads, 1) k_forces_adjoint(const float *po
     __shared__ double pe_s[kAThreads / 32];
     __shared__ float psum_s[3];
 
-    const int tid = threadIdx.x, p = tid & (kAP - 1), h = tid >> 7, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, p = tid & (kAP - 1), h = tid / kAP, warp = tid >> 5, lane = tid & 31;
     const int rs = 6 * npts + 1 - ((6 * npts) & 1);
     const int Kg = net.kin[0];
     const int first_limit = g_amlp_first_wait_limit;
@@ -553,8 +768,8 @@ __global__ void __launch_bounds__(kAThreads, 1) k_forces_adjoint(const float *po
     AdjShared S;
     size_t off = 0;
     // Two layouts. keep_r: the rotated points R have their own area and the
-    // descriptor partials g0, g1 live in the two operand tiles (free whenever
-    // the partials are), so R survives the net and is rotated once per tile.
+    // descriptor rows live in the first operand tile (free whenever the rows are
+    // live), so R survives the net and is rotated once per tile.
     // Otherwise (when that does not fit) R shares its area with the operand
     // tiles and is rotated again after the net.
     const size_t r_bytes = (size_t)kAP * rs * 4, ops_bytes = (size_t)2 * 2 * kAP * kWpad * 2;
@@ -573,29 +788,14 @@ __global__ void __launch_bounds__(kAThreads, 1) k_forces_adjoint(const float *po
     S.par = reinterpret_cast<float *>(smem_raw + off);
     off += align_up((size_t)net.par_total * 4, 128);
     if (keep_r) {
-        S.g0 = reinterpret_cast<float *>(op_tile(S.ops, 0));
-        S.g1 = reinterpret_cast<float *>(op_tile(S.ops, 1));
+        S.g = reinterpret_cast<float *>(op_tile(S.ops, 0));
     } else {
-        S.g0 = reinterpret_cast<float *>(smem_raw + off);
-        off += (size_t)kAP * DP * 4;
-        S.g1 = reinterpret_cast<float *>(smem_raw + off);
+        S.g = reinterpret_cast<float *>(smem_raw + off);
         off += (size_t)kAP * DP * 4;
     }
-    S.t = reinterpret_cast<float *>(smem_raw + off);
-    off += (size_t)kAP * 3 * 4;
-    S.cen = reinterpret_cast<float *>(smem_raw + off);
-    off += (size_t)kAP * 3 * 4;
-    S.part = reinterpret_cast<float *>(smem_raw + off);
-    off += (size_t)2 * kAP * kPartStride * 4;
-    S.eps = reinterpret_cast<float *>(smem_raw + off);
-    off += (size_t)2 * kAP * 4;
-    S.fd = reinterpret_cast<float *>(smem_raw + off);
-    off += (size_t)kAP * 9 * 4;
-    S.ij = reinterpret_cast<int *>(smem_raw + off);
-    off += (size_t)kAP * 2 * 4;
+    take_pair_areas<kAP>(S, smem_raw + off);
+    off += pair_area_bytes<kAP>();
     S.pts = reinterpret_cast<float *>(smem_raw + off);
-    off = align_up(off + (size_t)3 * npts * 4, 16);
-    S.q = reinterpret_cast<float4 *>(smem_raw + off);
     S.psum = psum_s;
 
     // ---- one-time set-up: weights (bf16 hi/lo, K-major), biases, TMEM, mbarrier
@@ -654,50 +854,35 @@ __global__ void __launch_bounds__(kAThreads, 1) k_forces_adjoint(const float *po
         phase ^= 1u;
         tc::fence_after();
     };
-
     const long long P = min(*d_np, cap);
     const long long ntiles = (P + kAP - 1) / kAP;
     double pe_acc = 0.0;
-    const int nd = 2 * npts;
 
     for (long long tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
         const long long p0 = tile * kAP;
         const int valid = (int)min((long long)kAP, P - p0);
         // ---- 1. pair indices, orientations, translations, then the rotated body points
-        if (tid < kAP) {
-            long long pr = min(p0 + tid, P - 1);
-            int i = pairs[2 * pr], j = pairs[2 * pr + 1];
-            S.q[2 * tid] = load_quat(quat, i);
-            S.q[2 * tid + 1] = load_quat(quat, j);
-            float dd;
-            float3 tt = min_image(pos, i, j, MULTI ? rp[rep[i]].box : L, &dd);
-            S.t[3 * tid] = tt.x;
-            S.t[3 * tid + 1] = tt.y;
-            S.t[3 * tid + 2] = tt.z;
-            S.ij[2 * tid] = i;
-            S.ij[2 * tid + 1] = j;
-            store_centroid(S, tid, npts);
-        }
-        __syncthreads();
-        rotate_tile(S, npts, rs);
+        load_pairs<kAP, MULTI>(S, pos, quat, L, pairs, P, p0, npts, rs, rep, rp);
         __syncthreads();
         // ---- 2. descriptor forward
         const float *Rp = S.R + p * rs;  // the pair's centred points
-        float A[Cfg::NA][KC];  // this half's sum_a f_n Y_k, kept in registers for the backward
-        if (h == 0) half_forward<Cfg, 0>(Rp, nd, inv_rc, S.g0 + p * DP, A);
-        else half_forward<Cfg, 1>(Rp, nd, inv_rc, S.g1 + p * DP, A);
+        float2 A[Cfg::NA][kHalfP];  // this half's sum_a f_n Y_k, kept in registers for the backward
+        if (h == 0) half_forward<Cfg, 0, kFusedUnroll>(Rp, npts, inv_rc, S.g + p * DP, A);
+        else half_forward<Cfg, 1, kFusedUnroll>(Rp, npts, inv_rc, S.g + p * DP, A);
+        __syncthreads();
+        if (h == 1) half_forward_finish<Cfg>(S.g + p * DP, A);
         __syncthreads();
         // ---- 3. net forward + backward on the tensor cores
         {
             char *tG = op_tile(S.ops, 0);
             // this thread's half of its row of g (kin[0] = 48 columns, set by the
             // launcher, 24 per half), read completely before the tile is written:
-            // with keep_r, g0 and g1 occupy the operand tiles
+            // with keep_r, the rows occupy the operand tile
             float v[24];
 #pragma unroll
             for (int k = 0; k < 24; ++k) {
                 int d = h * 24 + k;
-                v[k] = d < Cfg::D ? S.g0[p * DP + d] + S.g1[p * DP + d] : 0.f;
+                v[k] = S.g[p * DP + d];
             }
             __syncthreads();
 #pragma unroll
@@ -777,9 +962,9 @@ __global__ void __launch_bounds__(kAThreads, 1) k_forces_adjoint(const float *po
                 ++commits;
             }
             wait_mma();
+            const int cb = h * (Kp / 2), nch = Kp / 16;
             if (L2 > 0) {
                 char *dst = op_tile(S.ops, L2);
-                const int cb = h * (Kp / 2), nch = Kp / 16;
                 for (int ch = 0; ch < nch; ++ch) {  // a chunk of dz and of act'(z) per TMEM wait
                     const int c0 = cb + 8 * ch;
                     uint32_t r[16];
@@ -794,7 +979,6 @@ __global__ void __launch_bounds__(kAThreads, 1) k_forces_adjoint(const float *po
                 }
                 tc::fence_async_smem();
             } else {
-                const int cb = h * (Kp / 2), nch = Kp / 16;
                 for (int g = 0; g < nch; g += 2) {
                     float dg[2 * 8];
                     tc::tmem_ld8_many<2>(tmem + lane_base + bcol + cb + 8 * g, min(2, nch - g), dg);
@@ -802,115 +986,34 @@ __global__ void __launch_bounds__(kAThreads, 1) k_forces_adjoint(const float *po
                     for (int ch = 0; ch < 2; ++ch)
                         if (g + ch < nch)
 #pragma unroll
-                            for (int k = 0; k < 8; ++k) S.g0[p * DP + cb + 8 * (g + ch) + k] = dg[8 * ch + k];
+                            for (int k = 0; k < 8; ++k) S.g[p * DP + cb + 8 * (g + ch) + k] = dg[8 * ch + k];
                 }
             }
             tc::fence_before();
             aborted = __syncthreads_or(gave_up) != 0;
         }
         if (aborted) break;  // the net's outputs are not to be trusted: no forces from this tile
-        if (!MULTI && h == 0 && p < valid)
-            pe_acc += (double)en_min +
-                      (double)en_range * (double)(S.eps[p] + S.eps[kAP + p] + S.par[net.bias_off[net.nh] + kWpad]);
         // ---- 4. recompute the rotated points (their area held the MLP tiles)
         if (!keep_r) {
-            rotate_tile(S, npts, rs);
+            rotate_tile<kAP>(S, npts, rs);
             __syncthreads();
         }
         // ---- descriptor backward
-        if (h == 0) half_backward<Cfg, 0>(Rp, npts, inv_rc, S.g0 + p * DP, S.part + p * kPartStride, A);
-        else half_backward<Cfg, 1>(Rp, npts, inv_rc, S.g0 + p * DP, S.part + (kAP + p) * kPartStride, A);
+        float *part = S.part + (h * kAP + p) * kPartStride;
+        if (h == 0) half_backward<Cfg, 0>(Rp, npts, inv_rc, S.g + p * DP, part, A);
+        else half_backward<Cfg, 1>(Rp, npts, inv_rc, S.g + p * DP, part, A);
         __syncthreads();
-        // ---- 5. per-pair forces and torques
-        if (tid < kAP) {
-            const float *a0 = S.part + p * kPartStride, *a1 = S.part + (kAP + p) * kPartStride;
-            float Si[3], Sa[3], Xi[3], Xj[3];
-#pragma unroll
-            for (int k = 0; k < 3; ++k) {
-                Si[k] = a0[k] + a1[k];
-                Sa[k] = a0[3 + k] + a1[3 + k];
-                Xi[k] = a0[6 + k] + a1[6 + k];
-                Xj[k] = a0[9 + k] + a1[9 + k];
-            }
-            add_centroid_terms(S, p, Si, Sa, Xi, Xj);
-            // sums of the rotated points of i and of j: the rotation of the point sum
-            const float3 ps = make_float3(S.psum[0], S.psum[1], S.psum[2]);
-            const float3 pi3 = rotate_ref(S.q[2 * p], ps), qj3 = rotate_ref(S.q[2 * p + 1], ps);
-            const float Pi[3] = {pi3.x, pi3.y, pi3.z}, Qj[3] = {qj3.x, qj3.y, qj3.z};
-            const float inv_nd = 1.0f / (float)nd;
-            float Gm[3] = {Sa[0] * inv_nd, Sa[1] * inv_nd, Sa[2] * inv_nd};  // mean gradient
-            float Fp[3], Ti[3], Tj[3];
-#pragma unroll
-            for (int k = 0; k < 3; ++k) Fp[k] = -(Si[k] - (float)npts * Gm[k]);
-            Ti[0] = -(Xi[0] - (Pi[1] * Gm[2] - Pi[2] * Gm[1]));
-            Ti[1] = -(Xi[1] - (Pi[2] * Gm[0] - Pi[0] * Gm[2]));
-            Ti[2] = -(Xi[2] - (Pi[0] * Gm[1] - Pi[1] * Gm[0]));
-            Tj[0] = -(Xj[0] - (Qj[1] * Gm[2] - Qj[2] * Gm[1]));
-            Tj[1] = -(Xj[1] - (Qj[2] * Gm[0] - Qj[0] * Gm[2]));
-            Tj[2] = -(Xj[2] - (Qj[0] * Gm[1] - Qj[1] * Gm[0]));
-#pragma unroll
-            for (int k = 0; k < 3; ++k) {
-                S.fd[9 * p + k] = clip100(Fp[k] * en_range);
-                S.fd[9 * p + 3 + k] = clip100(Ti[k] * en_range);
-                S.fd[9 * p + 6 + k] = clip100(Tj[k] * en_range);
-            }
-        }
-        __syncthreads();
-        // ---- scatter: warps 0..3, lane = pair within a 32-pair group
-        if (warp < 4) {
-            const int q = warp * 32 + lane;
-            const bool ok = q < valid;
-            const int i = S.ij[2 * q], j = S.ij[2 * q + 1];
-            float v[6];
-#pragma unroll
-            for (int k = 0; k < 3; ++k) {
-                v[k] = ok ? S.fd[9 * q + k] : 0.f;
-                v[3 + k] = ok ? S.fd[9 * q + 3 + k] : 0.f;
-            }
-            if (ok) {
-#pragma unroll
-                for (int k = 0; k < 3; ++k) {
-                    atomicAdd(F + 3 * j + k, -v[k]);
-                    atomicAdd(T + 3 * j + k, S.fd[9 * q + 6 + k]);
-                }
-            }
-            const bool runs = warp_keys_sorted(i, ok);  // every lane takes part (warp vote)
-            int key = ok && runs ? i : -1 - q;  // unsorted pairs: no merging
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                int ko = __shfl_up_sync(0xffffffffu, key, o);
-#pragma unroll
-                for (int k = 0; k < 6; ++k) {
-                    float y = __shfl_up_sync(0xffffffffu, v[k], o);
-                    if (lane >= o && ko == key) v[k] += y;
-                }
-            }
-            int kn = __shfl_down_sync(0xffffffffu, key, 1);
-            if (ok && (lane == 31 || kn != key)) {
-#pragma unroll
-                for (int k = 0; k < 3; ++k) {
-                    atomicAdd(F + 3 * i + k, v[k]);
-                    atomicAdd(T + 3 * i + k, v[3 + k]);
-                }
-            }
-            if (MULTI && pe) {  // pair energies summed per system (systems own contiguous bodies)
-                double e = ok ? (double)en_min + (double)en_range *
-                                    (double)(S.eps[q] + S.eps[kAP + q] + S.par[net.bias_off[net.nh] + kWpad])
-                              : 0.0;
-                const int sys = ok ? rep[i] : 0;
-                const bool sys_runs = warp_keys_sorted(sys, ok);
-                int rk = ok && sys_runs ? sys : -1 - lane;
-#pragma unroll
-                for (int o = 1; o < 32; o <<= 1) {
-                    int ro = __shfl_up_sync(0xffffffffu, rk, o);
-                    double y = __shfl_up_sync(0xffffffffu, e, o);
-                    if (lane >= o && ro == rk) e += y;
-                }
-                int rn = __shfl_down_sync(0xffffffffu, rk, 1);
-                if (ok && (lane == 31 || rn != rk)) atomicAdd(pe + sys, e);
-            }
-        }
-        __syncthreads();
+        // ---- 5. per-pair forces and torques, scatter
+        const float b_last = S.par[net.bias_off[net.nh] + kWpad];
+        adj_finish_tile<kAP, MULTI>(
+            S, npts, valid, en_min, en_range,
+            [&](int q) { return S.eps[q] + S.eps[kAP + q] + b_last; }, F, T, pe, rep, pe_acc, 1);
+    }
+    if (aborted && tid == 0) {
+        atomicOr(&g_amlp_device_error, kErrMbarTimeout);
+        // the last MMA issued may still be in flight (thread 0 flipped `phase` after waiting for it):
+        // let it finish, with the normal limit, before TMEM is released
+        if (commits > 0) tc::mbar_wait(bar, phase ^ 1u, tc::kWaitLimit);
     }
     // ---- pair-energy sum, TMEM release
     if (!MULTI && pe) {
@@ -926,13 +1029,6 @@ __global__ void __launch_bounds__(kAThreads, 1) k_forces_adjoint(const float *po
         for (int k = 0; k < kAThreads / 32; ++k) s += pe_s[k];
         if (s != 0.0) atomicAdd(pe, s);
     }
-    if (aborted && tid == 0) {
-        atomicOr(&g_amlp_device_error, kErrMbarTimeout);
-        // the last MMA issued may still be in flight (thread 0 flipped `phase` after waiting for it):
-        // let it finish, with the normal limit, before TMEM is released
-        if (commits > 0) tc::mbar_wait(bar, phase ^ 1u, tc::kWaitLimit);
-    }
-    __syncthreads();
     if (warp == 0) {
         tc::fence_after();
         tc::tmem_dealloc(tmem, 512);
@@ -960,119 +1056,20 @@ constexpr int kGRow = 52;
 constexpr int kGP2 = 128;
 constexpr int kGRow2 = 132;
 constexpr size_t kWeightSplitBytes = (size_t)kMaxHiddenWide * kWideMax * kWideMax * 4;  // bf16 hi/lo, every layer
-constexpr size_t kAdjAFloats = 2 * 9 * 12;  // harmonic sums per pair kept between the passes (two halves of 9 x 12)
+constexpr size_t kAdjAFloats = 2 * 9 * kHalfK;  // harmonic sums per pair kept between the passes
 
 __host__ __device__ inline size_t adj_a_bytes(long long cap) {
-    return (size_t)((cap + 127) / 128) * 128 * kAdjAFloats * 4;
+    return (size_t)((cap + kDP - 1) / kDP) * kDP * kAdjAFloats * 4;
 }
 
-// Per-pair force/torque from the two halves' partial sums, scaled, clipped
-// (unless clip == 0), then scattered with runs of equal i summed in the warp
-// (warps 0..3, lane = pair).
-template <bool MULTI>
-__device__ __forceinline__ void adj_finish_tile(const AdjShared &S, int rs, int npts, int valid, float en_min,
-                                                float en_range, const float *y_rows, long long p0, float *F, float *T,
-                                                double *pe, const int *rep, double &pe_acc, int clip) {
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int nd = 2 * npts;
-    if (tid < kAP) {
-        const int p = tid;
-        const float *a0 = S.part + p * kPartStride, *a1 = S.part + (kAP + p) * kPartStride;
-        float Si[3], Sa[3], Xi[3], Xj[3];
-#pragma unroll
-        for (int k = 0; k < 3; ++k) {
-            Si[k] = a0[k] + a1[k];
-            Sa[k] = a0[3 + k] + a1[3 + k];
-            Xi[k] = a0[6 + k] + a1[6 + k];
-            Xj[k] = a0[9 + k] + a1[9 + k];
-        }
-        add_centroid_terms(S, p, Si, Sa, Xi, Xj);
-        const float3 ps = make_float3(S.psum[0], S.psum[1], S.psum[2]);
-        const float3 pi3 = rotate_ref(S.q[2 * p], ps), qj3 = rotate_ref(S.q[2 * p + 1], ps);
-        const float Pi[3] = {pi3.x, pi3.y, pi3.z}, Qj[3] = {qj3.x, qj3.y, qj3.z};
-        const float inv_nd = 1.0f / (float)nd;
-        float Gm[3] = {Sa[0] * inv_nd, Sa[1] * inv_nd, Sa[2] * inv_nd};
-        float Fp[3], Ti[3], Tj[3];
-#pragma unroll
-        for (int k = 0; k < 3; ++k) Fp[k] = -(Si[k] - (float)npts * Gm[k]);
-        Ti[0] = -(Xi[0] - (Pi[1] * Gm[2] - Pi[2] * Gm[1]));
-        Ti[1] = -(Xi[1] - (Pi[2] * Gm[0] - Pi[0] * Gm[2]));
-        Ti[2] = -(Xi[2] - (Pi[0] * Gm[1] - Pi[1] * Gm[0]));
-        Tj[0] = -(Xj[0] - (Qj[1] * Gm[2] - Qj[2] * Gm[1]));
-        Tj[1] = -(Xj[1] - (Qj[2] * Gm[0] - Qj[0] * Gm[2]));
-        Tj[2] = -(Xj[2] - (Qj[0] * Gm[1] - Qj[1] * Gm[0]));
-#pragma unroll
-        for (int k = 0; k < 3; ++k) {
-            float f = Fp[k] * en_range, ti = Ti[k] * en_range, tj = Tj[k] * en_range;
-            S.fd[9 * p + k] = clip ? clip100(f) : f;
-            S.fd[9 * p + 3 + k] = clip ? clip100(ti) : ti;
-            S.fd[9 * p + 6 + k] = clip ? clip100(tj) : tj;
-        }
-        if (!MULTI && p < valid) pe_acc += (double)en_min + (double)en_range * (double)y_rows[p0 + p];
-    }
-    __syncthreads();
-    if (warp < 4) {
-        const int q = warp * 32 + lane;
-        const bool ok = q < valid;
-        const int i = S.ij[2 * q], j = S.ij[2 * q + 1];
-        float v[6];
-#pragma unroll
-        for (int k = 0; k < 3; ++k) {
-            v[k] = ok ? S.fd[9 * q + k] : 0.f;
-            v[3 + k] = ok ? S.fd[9 * q + 3 + k] : 0.f;
-        }
-        if (ok) {
-#pragma unroll
-            for (int k = 0; k < 3; ++k) {
-                atomicAdd(F + 3 * j + k, -v[k]);
-                atomicAdd(T + 3 * j + k, S.fd[9 * q + 6 + k]);
-            }
-        }
-        const bool runs = warp_keys_sorted(i, ok);  // every lane takes part (warp vote)
-        int key = ok && runs ? i : -1 - q;  // unsorted pairs: no merging
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            int ko = __shfl_up_sync(0xffffffffu, key, o);
-#pragma unroll
-            for (int k = 0; k < 6; ++k) {
-                float yv = __shfl_up_sync(0xffffffffu, v[k], o);
-                if (lane >= o && ko == key) v[k] += yv;
-            }
-        }
-        int kn = __shfl_down_sync(0xffffffffu, key, 1);
-        if (ok && (lane == 31 || kn != key)) {
-#pragma unroll
-            for (int k = 0; k < 3; ++k) {
-                atomicAdd(F + 3 * i + k, v[k]);
-                atomicAdd(T + 3 * i + k, v[3 + k]);
-            }
-        }
-        if (MULTI && pe) {
-            double e = ok ? (double)en_min + (double)en_range * (double)y_rows[p0 + q] : 0.0;
-            const int sys = ok ? rep[i] : 0;
-            const bool sys_runs = warp_keys_sorted(sys, ok);
-            int rk = ok && sys_runs ? sys : -1 - lane;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                int ro = __shfl_up_sync(0xffffffffu, rk, o);
-                double yv = __shfl_up_sync(0xffffffffu, e, o);
-                if (lane >= o && ro == rk) e += yv;
-            }
-            int rn = __shfl_down_sync(0xffffffffu, rk, 1);
-            if (ok && (lane == 31 || rn != rk)) atomicAdd(pe + sys, e);
-        }
-    }
-    __syncthreads();
-}
-
-// dE/dg rows of the tile's pairs into S.g0 (row stride kGS), weighted by wt
+// dE/dg rows of the tile's pairs into S.g (row stride kGS), weighted by wt
 // when given; rows past `valid` are zero. One row per warp, lanes over columns.
 __device__ __forceinline__ void load_dg_rows(const AdjShared &S, const float *dg_rows, const float *wt, long long p0,
                                              int valid) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    for (int q = warp; q < kAP; q += kAThreads / 32) {
+    for (int q = warp; q < kDP; q += kDThreads / 32) {
         const float w = q < valid ? (wt ? wt[p0 + q] : 1.0f) : 0.f;
-        for (int d = lane; d < kGP; d += 32) S.g0[q * kGS + d] = q < valid ? w * dg_rows[(p0 + q) * kGP + d] : 0.f;
+        for (int d = lane; d < kGP; d += 32) S.g[q * kGS + d] = q < valid ? w * dg_rows[(p0 + q) * kGP + d] : 0.f;
     }
 }
 
@@ -1082,119 +1079,95 @@ __device__ __forceinline__ void load_dg_rows(const AdjShared &S, const float *dg
 // weights pair p's dE/dg by wt[p] (a vector-Jacobian product); clip = 0 turns
 // the +-100 clip of the per-pair forces and torques off.
 template <class Cfg, bool MULTI, bool BWD>
-__global__ void __launch_bounds__(kAThreads, 1) k_adj_desc(const float *pos, const float *quat, float L,
+__global__ void __launch_bounds__(kDThreads, 2) k_adj_desc(const float *pos, const float *quat, float L,
                                                           const int *pairs, const long long *d_np, long long cap,
                                                           const float *pts, int npts, float inv_rc, float en_min,
                                                           float en_range, float *g_rows, int g_ld,
                                                           const float *dg_rows, const float *y_rows, const float *wt,
                                                           int clip, float *F, float *T, double *pe, const int *rep,
                                                           const amlp_replica *rp, float *a_rows) {
-    constexpr int KC = Half<Cfg>::KC;
+    constexpr int KC = kHalfK;
     static_assert(2 * Cfg::NA * KC == kAdjAFloats, "harmonic sums per pair in the workspace");
     extern __shared__ __align__(128) char smem_raw[];
-    __shared__ double pe_s[kAThreads / 32];
+    __shared__ double pe_s[kDThreads / 32];
     __shared__ float psum_s[3];
-    const int tid = threadIdx.x, p = tid & (kAP - 1), h = tid >> 7, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, p = tid & (kDP - 1), h = tid / kDP, warp = tid >> 5, lane = tid & 31;
     const int rs = 6 * npts + 1 - ((6 * npts) & 1);
-    const int nd = 2 * npts;
     AdjShared S;
     S.psum = psum_s;
     size_t off = 0;
     S.R = reinterpret_cast<float *>(smem_raw);
-    off = align_up((size_t)kAP * rs * 4, 128);
-    S.g0 = reinterpret_cast<float *>(smem_raw + off);
-    off += (size_t)kAP * kGS * 4;
-    S.g1 = reinterpret_cast<float *>(smem_raw + off);
-    off += (size_t)kAP * kGS * 4;
-    S.t = reinterpret_cast<float *>(smem_raw + off);
-    off += (size_t)kAP * 3 * 4;
-    S.cen = reinterpret_cast<float *>(smem_raw + off);
-    off += (size_t)kAP * 3 * 4;
-    S.part = reinterpret_cast<float *>(smem_raw + off);
-    off += (size_t)2 * kAP * kPartStride * 4;
-    S.fd = reinterpret_cast<float *>(smem_raw + off);
-    off += (size_t)kAP * 9 * 4;
-    S.ij = reinterpret_cast<int *>(smem_raw + off);
-    off += (size_t)kAP * 2 * 4;
+    off = align_up((size_t)kDP * rs * 4, 128);
+    S.g = reinterpret_cast<float *>(smem_raw + off);
+    off += (size_t)kDP * kGS * 4;
+    take_pair_areas<kDP>(S, smem_raw + off);
+    off += pair_area_bytes<kDP>();
     S.pts = reinterpret_cast<float *>(smem_raw + off);
-    off = align_up(off + (size_t)3 * npts * 4, 16);
-    S.q = reinterpret_cast<float4 *>(smem_raw + off);
-    for (int k = tid; k < 3 * npts; k += kAThreads) S.pts[k] = pts[k];
+    for (int k = tid; k < 3 * npts; k += kDThreads) S.pts[k] = pts[k];
     __syncthreads();
     body_point_sum(S, npts);
     __syncthreads();
     const long long P = min(*d_np, cap);
-    const long long ntiles = (P + kAP - 1) / kAP;
+    const long long ntiles = (P + kDP - 1) / kDP;
     double pe_acc = 0.0;
     for (long long tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-        const long long p0 = tile * kAP;
-        const int valid = (int)min((long long)kAP, P - p0);
+        const long long p0 = tile * kDP;
+        const int valid = (int)min((long long)kDP, P - p0);
         // this thread's harmonic sums: computed by the forward pass (and stored
         // for the backward pass when a_rows is given), read back by the backward
         // pass; layout [tile][half][n][kk][pair] so that a warp's accesses coalesce
-        float A[Cfg::NA][KC];
-        float *a_tile = a_rows ? a_rows + ((size_t)tile * 2 + h) * (Cfg::NA * KC) * kAP + p : nullptr;
+        float2 A[Cfg::NA][kHalfP];
+        float *a_tile = a_rows ? a_rows + ((size_t)tile * 2 + h) * (Cfg::NA * KC) * kDP + p : nullptr;
         if (BWD && a_rows && tid == 0 && tile + gridDim.x < ntiles) {
             // the next tile's harmonic sums and dE/dg rows into L2 while this tile runs
             const long long nt = tile + gridDim.x;
-            const char *an = reinterpret_cast<const char *>(a_rows + (size_t)nt * 2 * (Cfg::NA * KC) * kAP);
-            constexpr uint32_t kABytes = 2u * Cfg::NA * KC * kAP * 4u, kPiece = 16384u;
+            const char *an = reinterpret_cast<const char *>(a_rows + (size_t)nt * 2 * (Cfg::NA * KC) * kDP);
+            constexpr uint32_t kABytes = 2u * Cfg::NA * KC * kDP * 4u, kPiece = 16384u;
             for (uint32_t o = 0; o < kABytes; o += kPiece) tc::bulk_prefetch_l2(an + o, min(kPiece, kABytes - o));
-            const uint32_t gb = (uint32_t)(min((long long)kAP, P - nt * kAP) * kGP * 4);
-            tc::bulk_prefetch_l2(dg_rows + nt * kAP * kGP, gb);
+            const uint32_t gb = (uint32_t)(min((long long)kDP, P - nt * kDP) * kGP * 4);
+            tc::bulk_prefetch_l2(dg_rows + nt * kDP * kGP, gb);
         }
         if (BWD && a_rows) {
             // the backward's inputs first, so that their loads overlap the rotation pass
 #pragma unroll
             for (int n = 0; n < Cfg::NA; ++n)
 #pragma unroll
-                for (int kk = 0; kk < KC; ++kk) A[n][kk] = a_tile[(n * KC + kk) * kAP];
+                for (int kk = 0; kk < KC; ++kk) pick(A[n], kk) = a_tile[(n * KC + kk) * kDP];
             load_dg_rows(S, dg_rows, wt, p0, valid);
         }
-        if (tid < kAP) {
-            long long pr = min(p0 + tid, P - 1);
-            int i = pairs[2 * pr], j = pairs[2 * pr + 1];
-            S.q[2 * tid] = load_quat(quat, i);
-            S.q[2 * tid + 1] = load_quat(quat, j);
-            float dd;
-            float3 tt = min_image(pos, i, j, MULTI ? rp[rep[i]].box : L, &dd);
-            S.t[3 * tid] = tt.x;
-            S.t[3 * tid + 1] = tt.y;
-            S.t[3 * tid + 2] = tt.z;
-            S.ij[2 * tid] = i;
-            S.ij[2 * tid + 1] = j;
-            store_centroid(S, tid, npts);
-        }
-        __syncthreads();
-        rotate_tile(S, npts, rs);
+        load_pairs<kDP, MULTI>(S, pos, quat, L, pairs, P, p0, npts, rs, rep, rp);
         __syncthreads();
         const float *Rp = S.R + p * rs;  // the pair's centred points
         if (!BWD || !a_rows) {
-            if (h == 0) half_forward<Cfg, 0>(Rp, nd, inv_rc, S.g0 + p * kGS, A);
-            else half_forward<Cfg, 1>(Rp, nd, inv_rc, S.g1 + p * kGS, A);
+            if (h == 0) half_forward<Cfg, 0, kWideUnroll>(Rp, npts, inv_rc, S.g + p * kGS, A);
+            else half_forward<Cfg, 1, kWideUnroll>(Rp, npts, inv_rc, S.g + p * kGS, A);
+            __syncthreads();
+            if (h == 1) half_forward_finish<Cfg>(S.g + p * kGS, A);
             if (!BWD && a_tile) {
 #pragma unroll
                 for (int n = 0; n < Cfg::NA; ++n)
 #pragma unroll
-                    for (int kk = 0; kk < KC; ++kk) a_tile[(n * KC + kk) * kAP] = A[n][kk];
+                    for (int kk = 0; kk < KC; ++kk) a_tile[(n * KC + kk) * kDP] = pick(A[n], kk);
             }
         }
         __syncthreads();
         if (!BWD) {
-            for (int q = warp; q < valid; q += kAThreads / 32)  // one row per warp: coalesced
+            for (int q = warp; q < valid; q += kDThreads / 32)  // one row per warp: coalesced
                 for (int d = lane; d < g_ld; d += 32)
-                    g_rows[(p0 + q) * g_ld + d] = d < Cfg::D ? S.g0[q * kGS + d] + S.g1[q * kGS + d] : 0.f;
+                    g_rows[(p0 + q) * g_ld + d] = d < Cfg::D ? S.g[q * kGS + d] : 0.f;
             __syncthreads();
             continue;
         }
-        if (!a_rows) {  // the forward partials held S.g0 until now
+        if (!a_rows) {  // the descriptor rows held S.g until now
             load_dg_rows(S, dg_rows, wt, p0, valid);
         }
         __syncthreads();
-        if (h == 0) half_backward<Cfg, 0>(Rp, npts, inv_rc, S.g0 + p * kGS, S.part + p * kPartStride, A);
-        else half_backward<Cfg, 1>(Rp, npts, inv_rc, S.g0 + p * kGS, S.part + (kAP + p) * kPartStride, A);
+        float *part = S.part + (h * kDP + p) * kPartStride;
+        if (h == 0) half_backward<Cfg, 0>(Rp, npts, inv_rc, S.g + p * kGS, part, A);
+        else half_backward<Cfg, 1>(Rp, npts, inv_rc, S.g + p * kGS, part, A);
         __syncthreads();
-        adj_finish_tile<MULTI>(S, rs, npts, valid, en_min, en_range, y_rows, p0, F, T, pe, rep, pe_acc, clip);
+        adj_finish_tile<kDP, MULTI>(
+            S, npts, valid, en_min, en_range, [&](int q) { return y_rows[p0 + q]; }, F, T, pe, rep, pe_acc, clip);
     }
     if (BWD && !MULTI && pe) {
         double v = pe_acc;
@@ -1204,7 +1177,7 @@ __global__ void __launch_bounds__(kAThreads, 1) k_adj_desc(const float *pos, con
         __syncthreads();
         if (tid == 0) {
             double s = 0.0;
-            for (int k = 0; k < kAThreads / 32; ++k) s += pe_s[k];
+            for (int k = 0; k < kDThreads / 32; ++k) s += pe_s[k];
             if (s != 0.0) atomicAdd(pe, s);
         }
     }
@@ -1537,18 +1510,18 @@ static amlp_status launch_adjoint(const float *d_pos, const float *d_quat, float
     net.par_total = par;
     const int npts = nep->npts;
     const int rs = 6 * npts + 1 - ((6 * npts) & 1);
-    size_t r_bytes = (size_t)kAP * rs * 4, ops_bytes = (size_t)2 * 2 * kAP * kWpad * 2;
-    static_assert((size_t)kAP * kGS * 4 <= (size_t)2 * kAP * kWpad * 2, "descriptor partials fit an operand tile");
-    const size_t tail = (size_t)kAP * 3 * 4 * 2 + (size_t)2 * kAP * kPartStride * 4 + (size_t)2 * kAP * 4 +
-                        (size_t)kAP * 9 * 4 + (size_t)kAP * 2 * 4 + (size_t)3 * npts * 4 + (size_t)kAP * 32 + 16 + 128;
+    const size_t r_bytes = align_up((size_t)kAP * rs * 4, 128), ops_bytes = (size_t)2 * 2 * kAP * kWpad * 2;
+    static_assert((size_t)kAP * kGS * 4 <= (size_t)2 * kAP * kWpad * 2, "descriptor rows fit an operand tile");
+    const size_t tail = align_up(wsm, 128) + align_up((size_t)par * 4, 128) + pair_area_bytes<kAP>() +
+                        (size_t)3 * npts * 4 + 16 + 128;
     // R kept apart from the operand tiles (one rotation pass per tile) when it fits
-    const size_t smem_keep = align_up(r_bytes, 128) + align_up(ops_bytes, 128) + align_up(wsm, 128) +
-                             align_up((size_t)par * 4, 128) + tail;
-    const size_t smem_shared = align_up(std::max(r_bytes, ops_bytes), 128) + align_up(wsm, 128) +
-                               align_up((size_t)par * 4, 128) + (size_t)kAP * kGS * 4 * 2 + tail;
+    const size_t row_bytes = (size_t)kAP * kGS * 4;
+    const size_t smem_keep = r_bytes + ops_bytes + tail;
+    const size_t smem_shared = std::max(r_bytes, ops_bytes) + row_bytes + tail;
     const int keep_r = smem_keep <= 220 * 1024 ? 1 : 0;
     const size_t smem = keep_r ? smem_keep : smem_shared;
-    if (smem > 220 * 1024) return AMLP_ERR_UNSUPPORTED;
+    // the shapes and nets taken: those that leave room for a second copy of the rows
+    if (smem + (keep_r ? 0 : row_bytes) > 220 * 1024) return AMLP_ERR_UNSUPPORTED;
     using Cfg = NepCfg<10, 8, 4, 12>;
     cudaStream_t s = as_stream(stream);
     const float inv_rc = 1.0f / nep->nep_cutoff, rng = nep->en_max - nep->en_min;
@@ -1646,11 +1619,12 @@ extern "C" amlp_status amlp_adjoint_workspace_bytes(long long cap, size_t *bytes
     return AMLP_OK;
 }
 
+// Body points the harmonic descriptor passes take (at 48, 115 KB of shared memory per block).
+constexpr int kHarmonicMaxPts = 48;
 static size_t wide_desc_smem(int npts) {
     const int rs = 6 * npts + 1 - ((6 * npts) & 1);
-    return align_up((size_t)kAP * rs * 4, 128) + (size_t)kAP * kGS * 4 * 2 + (size_t)kAP * 3 * 4 * 2 +
-           (size_t)2 * kAP * kPartStride * 4 + (size_t)kAP * 9 * 4 + (size_t)kAP * 2 * 4 + (size_t)3 * npts * 4 +
-           (size_t)kAP * 32 + 16;
+    return align_up((size_t)kDP * rs * 4, 128) + (size_t)kDP * kGS * 4 + pair_area_bytes<kDP>() +
+           (size_t)3 * npts * 4;
 }
 
 static amlp_status check_pair_args(const float *d_pos, const float *d_quat, const int *d_pairs,
@@ -1754,7 +1728,7 @@ static amlp_status launch_adjoint_wide(const float *d_pos, const float *d_quat, 
     const int npts = nep->npts;
     const size_t smem_desc = wide_desc_smem(npts);
     const size_t smem_mlp = (size_t)net.smem;
-    if (smem_desc > 220 * 1024) return AMLP_ERR_UNSUPPORTED;
+    if (npts > kHarmonicMaxPts) return AMLP_ERR_UNSUPPORTED;
     using Cfg = NepCfg<10, 8, 4, 12>;
     const bool multi = d_rep != nullptr;
     auto fwd = multi ? k_adj_desc<Cfg, true, false> : k_adj_desc<Cfg, false, false>;
@@ -1763,14 +1737,14 @@ static amlp_status launch_adjoint_wide(const float *d_pos, const float *d_quat, 
     AMLP_CHECK_CUDA(cudaFuncSetAttribute(bwd, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_desc));
     AMLP_CHECK_CUDA(cudaFuncSetAttribute(k_mlp_grad, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_mlp));
     stage_mark(0, s);
-    fwd<<<kNumSM, kAThreads, smem_desc, s>>>(d_pos, d_quat, box, d_pairs, d_npairs, cap, nep->d_pts, npts, inv_rc,
+    fwd<<<2 * kNumSM, kDThreads, smem_desc, s>>>(d_pos, d_quat, box, d_pairs, d_npairs, cap, nep->d_pts, npts, inv_rc,
                                              nep->en_min, rng, g_rows, kGRow, nullptr, nullptr, nullptr, clip, d_F,
                                              d_T, d_pe, d_rep, d_rp, a_rows);
     stage_mark(1, s);
     k_split_weights<<<64, 256, 0, s>>>(net, mlp->d_w, wsplit);
     k_mlp_grad<<<kNumSM, kMThreads, smem_mlp, s>>>(g_rows, d_npairs, cap, net, mlp->d_w, wsplit, y_rows, dg_rows);
     stage_mark(2, s);
-    bwd<<<kNumSM, kAThreads, smem_desc, s>>>(d_pos, d_quat, box, d_pairs, d_npairs, cap, nep->d_pts, npts, inv_rc,
+    bwd<<<2 * kNumSM, kDThreads, smem_desc, s>>>(d_pos, d_quat, box, d_pairs, d_npairs, cap, nep->d_pts, npts, inv_rc,
                                              nep->en_min, rng, nullptr, kGP, dg_rows, y_rows, d_wt, clip, d_F, d_T,
                                              d_pe, d_rep, d_rp, a_rows);
     stage_mark(3, s);
@@ -1818,11 +1792,11 @@ extern "C" amlp_status amlp_pair_descriptors(const float *d_pos, const float *d_
         return check_launch();
     }
     const size_t smem = wide_desc_smem(nep->npts);
-    if (smem > 220 * 1024) return AMLP_ERR_UNSUPPORTED;
+    if (nep->npts > kHarmonicMaxPts) return AMLP_ERR_UNSUPPORTED;
     using Cfg = NepCfg<10, 8, 4, 12>;
     auto fwd = k_adj_desc<Cfg, false, false>;
     AMLP_CHECK_CUDA(cudaFuncSetAttribute(fwd, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    fwd<<<kNumSM, kAThreads, smem, as_stream(stream)>>>(d_pos, d_quat, box, d_pairs, d_npairs, cap, nep->d_pts,
+    fwd<<<2 * kNumSM, kDThreads, smem, as_stream(stream)>>>(d_pos, d_quat, box, d_pairs, d_npairs, cap, nep->d_pts,
                                                         nep->npts, 1.0f / nep->nep_cutoff, nep->en_min,
                                                         nep->en_max - nep->en_min, d_g, ld_g, nullptr, nullptr,
                                                         nullptr, 1, nullptr, nullptr, nullptr, nullptr, nullptr,
