@@ -81,6 +81,26 @@ __device__ __forceinline__ float act_df(int act, float z) {
     return s * (1.0f + z * (1.0f - s));
 }
 
+// Two FP32 multiply-adds in one instruction, each rounded as fmaf. The pair takes
+// the multiply-add pipe as long as two, but one issue slot, which leaves the other
+// slot to the loads and address arithmetic of a register-tiled product.
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+    unsigned long long d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;"
+        : "=l"(d)
+        : "l"(*reinterpret_cast<unsigned long long *>(&a)), "l"(*reinterpret_cast<unsigned long long *>(&b)),
+          "l"(*reinterpret_cast<unsigned long long *>(&c)));
+    return *reinterpret_cast<float2 *>(&d);
+}
+
+// 1 / sqrt(x) to the same two ulp as rsqrtf, without its handling of
+// subnormal arguments (a squared distance is 0 or far above them).
+__device__ __forceinline__ float rsqrt_ftz(float x) {
+    float r;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+
 // True when the keys of the valid lanes never decrease from one lane to the
 // next, so that equal keys form contiguous runs and a segmented warp sum over
 // runs is exact. `ok` marks the valid lanes, a prefix of the warp. Pair lists

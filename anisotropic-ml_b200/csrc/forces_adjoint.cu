@@ -152,25 +152,8 @@ __host__ __device__ constexpr float half_scale(int H, int kk) {
     return t[H][kk];
 }
 
-// Two FP32 multiply-adds in one instruction, each rounded as fmaf.
-__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
-    unsigned long long d;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;"
-        : "=l"(d)
-        : "l"(*reinterpret_cast<unsigned long long *>(&a)), "l"(*reinterpret_cast<unsigned long long *>(&b)),
-          "l"(*reinterpret_cast<unsigned long long *>(&c)));
-    return *reinterpret_cast<float2 *>(&d);
-}
 // Element kk of an array of pairs (kk a constant after unrolling).
 __device__ __forceinline__ float &pick(float2 *v, int kk) { return kk & 1 ? v[kk >> 1].y : v[kk >> 1].x; }
-
-// 1 / sqrt(x) to the same two ulp as rsqrtf, without its handling of
-// subnormal arguments (a squared distance is 0 or far above them).
-__device__ __forceinline__ float rsqrt_ftz(float x) {
-    float r;
-    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
-    return r;
-}
 
 // T_1 .. T_N of x, t[n] = T_n (t[0] unused).
 template <int N>

@@ -5,120 +5,366 @@
 //   L = (1/B) sum_r (net(g_r) - y_r)^2.
 // The same kernel also backpropagates a given per-row upstream gradient dy_r
 // (a vector-Jacobian product, sum_r dy_r d net(g_r) / d theta).
-// Backpropagation into every weight and bias, FP32. A CTA takes 32 rows: the
-// forward keeps pre-activations and activations of its rows in shared memory,
-// the backward forms the deltas and adds its rows' share of dL/dW and dL/db to
-// the caller's gradient buffer (one atomic per weight per CTA).
+// Backpropagation into every weight and bias, FP32.
+//
+// A CTA keeps all activations of a tile of R rows in shared memory, feature-major
+// (a feature's R values contiguous), and runs the three products of every layer on
+// them as register tiles:
+//   forward   z[r][n]  = b[n] + sum_k W[n][k] a[r][k]  (ascending k, one rounding per
+//             multiply-add), thread = 4 rows x NC columns;
+//   gradient  dW[n][k] = sum_r delta[r][n] a[r][k], thread = NJ x NI weights over all
+//             rows, a warp's lanes on consecutive k: one coalesced reduction per
+//             weight and tile into the caller's gradient buffer;
+//   deltas    delta_prev[r][k] = act' sum_n W[n][k] delta[r][n], thread as forward,
+//             written over the activations they belong to (ReLU's and tanh's
+//             derivatives follow from the activation; SiLU keeps z beside it).
+// The weights are read through L1 (a warp shares each of them), so that the shared
+// memory holds rows alone: the more rows per tile, the fewer reductions. R is
+// chosen so that the tiles fill whole rounds of the SMs, at most 64.
+// Bound by the L1 that serves both the rows and the weights (72 % of its rate, the
+// multiply-add pipe at 35 %). 16,384 rows of the 47-150-150-150-150-1 ReLU net: 347 us,
+// 21 TFLOP/s. Before, 3,254 us: a thread walked one output column over 32 rows with a
+// shared-memory load per multiply-add, and every 32 rows paid one reduction per weight.
+#include <algorithm>
+
 #include "common.cuh"
 
 namespace amlp {
 namespace {
 
-constexpr int kTrainRows = 32;
-constexpr int kTrainThreads = 128;
+constexpr int kTrainThreads = 512;
+constexpr int kTrainMaxRows = 64;
 constexpr int kTrainMaxWidth = 256;
+constexpr size_t kTrainSmem = 226 * 1024;
 
 struct TrainNet {
     int n_layers, act;
     int dims[AMLP_MAX_LAYERS + 1];
     long long woff[AMLP_MAX_LAYERS];
-    int aoff[AMLP_MAX_LAYERS + 1];  // float offset of layer k's activations (rows x dims[k]) in smem
-    int total;                      // floats of activations (and as many for pre-activations / deltas)
+    int feat[AMLP_MAX_LAYERS + 1];  // first feature of layer k's activations (then deltas)
+    int zfeat[AMLP_MAX_LAYERS + 1]; // SiLU: first feature of layer k's pre-activations
+    int rg, ld;                     // row groups of 4 per tile, floats per feature
 };
 
-__global__ void __launch_bounds__(kTrainThreads) k_mlp_loss_grad(const float *g, const float *y, const float *dy,
-                                                                 long long rows, TrainNet net, const float *w,
-                                                                 float *grad, double *loss) {
-    extern __shared__ float sm[];
-    float *act = sm;               // activations a_k[r][i], k = 0..n_layers (a_0 = g)
-    float *pre = sm + net.total;   // pre-activations z_k (k >= 1), then deltas in place
-    const int tid = threadIdx.x;
-    const float inv_b = 1.0f / (float)rows;
-    for (long long r0 = (long long)blockIdx.x * kTrainRows; r0 < rows; r0 += (long long)gridDim.x * kTrainRows) {
-        const int nr = (int)min((long long)kTrainRows, rows - r0);
-        const int D = net.dims[0];
-        for (int idx = tid; idx < kTrainRows * D; idx += kTrainThreads) {
-            int r = idx / D, d = idx - r * D;
-            act[net.aoff[0] + idx] = r < nr ? g[(r0 + r) * D + d] : 0.f;
+// Features are ld floats apart: ld / 4 is odd, so that 8 lanes' 16-byte reads of
+// consecutive features fall in distinct bank groups.
+__host__ __device__ constexpr int train_ld(int rg) { return 4 * (rg | 1); }
+
+// acc[i][c] (rows 2 i, 2 i + 1) += sum over k = 0 .. K - 1, ascending, of x[k][rows]
+// times the weight of column c: x points at the thread's four rows of feature 0
+// (features ld apart). ROWS: column c's weights are consecutive floats at w + c col
+// (the forward's, one row of W per column; vec2: 8-byte aligned), otherwise the
+// columns are consecutive and k's weights are the floats at w + k step (the
+// deltas', one row of W per k). The next four k's weights load while four k's
+// multiply-adds issue.
+template <int NC, bool ROWS>
+__device__ __forceinline__ void train_product(float2 (&acc)[2][NC], const float *x, int ld, int K, const float *w,
+                                              int col, int step, bool vec2) {
+    const float *p[ROWS ? NC : 1];
+    p[0] = w;
+    if (ROWS) {
+#pragma unroll
+        for (int c = 1; c < NC; ++c) p[c] = w + c * col;
+    }
+    auto mul = [&](const float4 &xv, const float (&wv)[NC]) {
+#pragma unroll
+        for (int c = 0; c < NC; ++c) {
+            acc[0][c] = fma2(make_float2(xv.x, xv.y), make_float2(wv[c], wv[c]), acc[0][c]);
+            acc[1][c] = fma2(make_float2(xv.z, xv.w), make_float2(wv[c], wv[c]), acc[1][c]);
         }
-        __syncthreads();
-        // forward
-        for (int L = 0; L < net.n_layers; ++L) {
-            const int K = net.dims[L], N = net.dims[L + 1];
-            const float *W = w + net.woff[L], *b = W + (size_t)N * K;
-            const bool last = L == net.n_layers - 1;
-            for (int n = tid; n < N; n += kTrainThreads) {
-                float acc[kTrainRows];
+    };
+    auto load1 = [&](float (&wv)[NC]) {  // the next k's weights
 #pragma unroll
-                for (int r = 0; r < kTrainRows; ++r) acc[r] = __ldg(b + n);
-                for (int k = 0; k < K; ++k) {
-                    float wv = __ldg(W + (size_t)n * K + k);
+        for (int c = 0; c < NC; ++c) wv[c] = ROWS ? __ldg(p[c]) : __ldg(p[0] + c);
+        if (ROWS) {
 #pragma unroll
-                    for (int r = 0; r < kTrainRows; ++r) acc[r] = fmaf(wv, act[net.aoff[L] + r * K + k], acc[r]);
+            for (int c = 0; c < NC; ++c) ++p[c];
+        } else {
+            p[0] += step;
+        }
+    };
+    auto load4 = [&](float (&wv)[4][NC]) {
+        if (ROWS && vec2) {
+#pragma unroll
+            for (int c = 0; c < NC; ++c) {
+                const float2 a = __ldg(reinterpret_cast<const float2 *>(p[c]));
+                const float2 b = __ldg(reinterpret_cast<const float2 *>(p[c]) + 1);
+                wv[0][c] = a.x, wv[1][c] = a.y, wv[2][c] = b.x, wv[3][c] = b.y;
+                p[c] += 4;
+            }
+        } else {
+#pragma unroll
+            for (int u = 0; u < 4; ++u) load1(wv[u]);
+        }
+    };
+    int k = 0;
+    if (K >= 4) {
+        float cur[4][NC];
+        load4(cur);
+#pragma unroll 1
+        for (k = 4; k + 4 <= K; k += 4, x += 4 * ld) {
+            float nxt[4][NC];
+            load4(nxt);
+#pragma unroll
+            for (int u = 0; u < 4; ++u) mul(*reinterpret_cast<const float4 *>(x + u * ld), cur[u]);
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+#pragma unroll
+                for (int c = 0; c < NC; ++c) cur[u][c] = nxt[u][c];
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) mul(*reinterpret_cast<const float4 *>(x + u * ld), cur[u]);
+        x += 4 * ld;
+    }
+#pragma unroll 1
+    for (; k < K; ++k, x += ld) {
+        float wv[NC];
+        load1(wv);
+        mul(*reinterpret_cast<const float4 *>(x), wv);
+    }
+}
+
+// Consecutive columns per thread of a layer of n, ncg column groups: 1 to 5, or two
+// groups of 4.
+__device__ __forceinline__ int train_columns(int n, int ncg) {
+    const int nc = (n + ncg - 1) / ncg;
+    return nc > 5 ? 8 : nc;
+}
+
+// First of a thread's NC consecutive columns from c0, moved back so that all lie
+// below n (the columns below c0 then belong to another thread).
+__device__ __forceinline__ int train_first(int c0, int nc, int n) { return max(0, min(c0, n - nc)); }
+
+struct TrainTile {
+    float *sm;
+    int tid, rg, cg, ncg;  // row group (4 rows), column group and their number
+    bool on;               // threads past the last whole column group idle in the products
+};
+
+// Layer L forward for NC columns per thread from n0.
+template <int NC>
+__device__ __forceinline__ void train_forward(const TrainNet &net, const TrainTile &t, const float *wts, int L,
+                                              int n0) {
+    const int K = net.dims[L], N = net.dims[L + 1], ld = net.ld;
+    const float *W = wts + net.woff[L], *b = W + (size_t)N * K;
+    const bool last = L == net.n_layers - 1;
+    const int f = train_first(n0, NC, N);
+    float2 acc[2][NC];
+#pragma unroll
+    for (int c = 0; c < NC; ++c) {
+        const float bv = __ldg(b + f + c);
+        acc[0][c] = acc[1][c] = make_float2(bv, bv);
+    }
+    const bool vec2 = (K & 1) == 0 && (reinterpret_cast<uintptr_t>(W) & 7) == 0;
+    train_product<NC, true>(acc, t.sm + net.feat[L] * ld + 4 * t.rg, ld, K, W + (size_t)f * K, K, 0, vec2);
+#pragma unroll
+    for (int c = 0; c < NC; ++c) {
+        const int n = f + c;
+        if (n < n0) continue;
+        const float z[4] = {acc[0][c].x, acc[0][c].y, acc[1][c].x, acc[1][c].y};
+        float a[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) a[i] = last ? z[i] : act_f(net.act, z[i]);
+        *reinterpret_cast<float4 *>(t.sm + (net.feat[L + 1] + n) * ld + 4 * t.rg) = make_float4(a[0], a[1], a[2], a[3]);
+        if (!last && net.act == AMLP_ACT_SILU)
+            *reinterpret_cast<float4 *>(t.sm + (net.zfeat[L + 1] + n) * ld + 4 * t.rg) =
+                make_float4(z[0], z[1], z[2], z[3]);
+    }
+}
+
+// The deltas of layer L's inputs without act', for NC columns per thread from
+// train_first(k0, NC, K), into out.
+template <int NC>
+__device__ __forceinline__ void train_deltas(const TrainNet &net, const TrainTile &t, const float *wts, int L, int k0,
+                                             float4 *out) {
+    const int K = net.dims[L], N = net.dims[L + 1], ld = net.ld;
+    const float *W = wts + net.woff[L];
+    float2 acc[2][NC];
+#pragma unroll
+    for (int c = 0; c < NC; ++c) acc[0][c] = acc[1][c] = make_float2(0.f, 0.f);
+    train_product<NC, false>(acc, t.sm + net.feat[L + 1] * ld + 4 * t.rg, ld, N, W + train_first(k0, NC, K), 0, K,
+                             false);
+#pragma unroll
+    for (int c = 0; c < NC; ++c) out[c] = make_float4(acc[0][c].x, acc[0][c].y, acc[1][c].x, acc[1][c].y);
+}
+
+// act' times the delta d of the thread's rows of feature k, over the activations.
+__device__ __forceinline__ void train_store_delta(const TrainNet &net, const TrainTile &t, int L, int k, float4 dv) {
+    float4 *dst = reinterpret_cast<float4 *>(t.sm + (net.feat[L] + k) * net.ld + 4 * t.rg);
+    const float4 av = *dst;
+    const float a[4] = {av.x, av.y, av.z, av.w};
+    float d[4] = {dv.x, dv.y, dv.z, dv.w};
+    if (net.act == AMLP_ACT_SILU) {
+        const float4 zv = *reinterpret_cast<const float4 *>(t.sm + (net.zfeat[L] + k) * net.ld + 4 * t.rg);
+        const float z[4] = {zv.x, zv.y, zv.z, zv.w};
+#pragma unroll
+        for (int i = 0; i < 4; ++i) d[i] *= act_df(AMLP_ACT_SILU, z[i]);
+    } else if (net.act == AMLP_ACT_TANH) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) d[i] *= 1.0f - a[i] * a[i];
+    } else {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) d[i] *= a[i] > 0.0f ? 1.0f : 0.0f;
+    }
+    *dst = make_float4(d[0], d[1], d[2], d[3]);
+}
+
+// dL/dW of layer L from its deltas and inputs: warp w takes rows
+// n = w, w + 16, ... of W, NJ at a time, its lanes the columns
+// k = k0 + lane + 32 i.
+template <int NI>
+__device__ __forceinline__ void train_weights(const TrainNet &net, const TrainTile &t, float *grad, int L, int k0) {
+    constexpr int NJ = 5, nw = kTrainThreads / 32;
+    const int K = net.dims[L], N = net.dims[L + 1], ld = net.ld, R = 4 * net.rg;
+    const int warp = t.tid >> 5, lane = t.tid & 31;
+    float *gW = grad + net.woff[L];
+    const float *a[NI];
+#pragma unroll
+    for (int i = 0; i < NI; ++i) a[i] = t.sm + (net.feat[L] + min(k0 + lane + 32 * i, K - 1)) * ld;
+#pragma unroll 1
+    for (int n0 = warp; n0 < N; n0 += nw * NJ) {
+        const float *d[NJ];
+        float2 acc[NJ][NI];
+#pragma unroll
+        for (int j = 0; j < NJ; ++j) {
+            d[j] = t.sm + (net.feat[L + 1] + min(n0 + nw * j, N - 1)) * ld;
+#pragma unroll
+            for (int i = 0; i < NI; ++i) acc[j][i] = make_float2(0.f, 0.f);
+        }
+#pragma unroll 1
+        for (int r = 0; r < R; r += 4) {
+            float4 av[NI];
+#pragma unroll
+            for (int i = 0; i < NI; ++i) av[i] = *reinterpret_cast<const float4 *>(a[i] + r);
+#pragma unroll
+            for (int j = 0; j < NJ; ++j) {
+                const float4 dv = *reinterpret_cast<const float4 *>(d[j] + r);
+#pragma unroll
+                for (int i = 0; i < NI; ++i) {
+                    acc[j][i] = fma2(make_float2(dv.x, dv.y), make_float2(av[i].x, av[i].y), acc[j][i]);
+                    acc[j][i] = fma2(make_float2(dv.z, dv.w), make_float2(av[i].z, av[i].w), acc[j][i]);
                 }
+            }
+        }
 #pragma unroll
-                for (int r = 0; r < kTrainRows; ++r) {
-                    pre[net.aoff[L + 1] + r * N + n] = acc[r];
-                    act[net.aoff[L + 1] + r * N + n] = last ? acc[r] : act_f(net.act, acc[r]);
+        for (int j = 0; j < NJ; ++j) {
+            const int n = n0 + nw * j;
+            if (n >= N) break;
+#pragma unroll
+            for (int i = 0; i < NI; ++i) {
+                const int k = k0 + lane + 32 * i;
+                if (k < K) atomicAdd(gW + (size_t)n * K + k, acc[j][i].x + acc[j][i].y);
+            }
+        }
+    }
+}
+
+// dL/db of layer L.
+__device__ __forceinline__ void train_bias(const TrainNet &net, const TrainTile &t, float *grad, int L) {
+    const int K = net.dims[L], N = net.dims[L + 1], ld = net.ld, R = 4 * net.rg;
+    float *gb = grad + net.woff[L] + (size_t)N * K;
+    for (int n = t.tid; n < N; n += kTrainThreads) {
+        const float *d = t.sm + (net.feat[L + 1] + n) * ld;
+        float s = 0.f;
+        for (int r = 0; r < R; r += 4) {
+            const float4 v = *reinterpret_cast<const float4 *>(d + r);
+            s += (v.x + v.y) + (v.z + v.w);
+        }
+        atomicAdd(gb + n, s);
+    }
+}
+
+__global__ void __launch_bounds__(kTrainThreads, 1) k_mlp_loss_grad(const float *g, const float *y, const float *dy,
+                                                                    long long rows, TrainNet net, const float *w,
+                                                                    float *grad, double *loss) {
+    extern __shared__ __align__(16) float sm[];
+    const int ld = net.ld, R = 4 * net.rg;
+    TrainTile t;
+    t.sm = sm;
+    t.tid = threadIdx.x;
+    t.ncg = kTrainThreads / net.rg;
+    t.cg = t.tid / net.rg;
+    t.rg = t.tid - t.cg * net.rg;
+    t.on = t.cg < t.ncg;
+    const float inv_b = 1.0f / (float)rows;
+    for (long long r0 = (long long)blockIdx.x * R; r0 < rows; r0 += (long long)gridDim.x * R) {
+        const int nr = (int)min((long long)R, rows - r0);
+        const int D = net.dims[0];
+        // the tile's descriptor rows, a warp per row (coalesced); rows past the end are zero
+        for (int r = t.tid >> 5; r < R; r += kTrainThreads / 32)
+            for (int d = t.tid & 31; d < D; d += 32) sm[d * ld + r] = r < nr ? g[(r0 + r) * D + d] : 0.f;
+        __syncthreads();
+        for (int L = 0; L < net.n_layers; ++L) {
+            if (t.on) {
+                // nc consecutive columns per thread
+                const int N = net.dims[L + 1], nc = train_columns(N, t.ncg), n0 = t.cg * nc;
+                if (n0 < N) {
+                    if (nc == 8) {
+                        train_forward<4>(net, t, w, L, n0);
+                        if (n0 + 4 < N) train_forward<4>(net, t, w, L, n0 + 4);
+                    } else if (nc == 5) train_forward<5>(net, t, w, L, n0);
+                    else if (nc == 4) train_forward<4>(net, t, w, L, n0);
+                    else if (nc == 3) train_forward<3>(net, t, w, L, n0);
+                    else if (nc == 2) train_forward<2>(net, t, w, L, n0);
+                    else train_forward<1>(net, t, w, L, n0);
                 }
             }
             __syncthreads();
         }
         // output delta: dy, or dL/dz_last = 2 (net - y) / B and the loss
-        const int Ll = net.n_layers;
-        if (tid < kTrainRows) {
+        if (t.tid < kTrainMaxRows) {
+            float *out = sm + net.feat[net.n_layers] * ld + t.tid;
             float d = 0.f;
             double l = 0.0;
-            if (tid < nr && dy) {
-                d = dy[r0 + tid];
-            } else if (tid < nr) {
-                float e = act[net.aoff[Ll] + tid] - y[r0 + tid];
+            if (t.tid < nr && dy) {
+                d = dy[r0 + t.tid];
+            } else if (t.tid < nr) {
+                float e = *out - y[r0 + t.tid];
                 d = 2.0f * e * inv_b;
                 l = (double)e * (double)e / (double)rows;
             }
-            pre[net.aoff[Ll] + tid] = d;
+            if (t.tid < R) *out = d;
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1) l += __shfl_xor_sync(0xffffffffu, l, o);
-            if (tid == 0 && loss) atomicAdd(loss, l);
+            if ((t.tid & 31) == 0 && loss && l != 0.0) atomicAdd(loss, l);
         }
         __syncthreads();
-        // backward: delta_L (rows x N) in pre[aoff[L+1]]
         for (int L = net.n_layers - 1; L >= 0; --L) {
-            const int K = net.dims[L], N = net.dims[L + 1];
-            const float *W = w + net.woff[L];
-            float *gW = grad + net.woff[L], *gb = gW + (size_t)N * K;
-            const float *delta = pre + net.aoff[L + 1];
-            const float *a = act + net.aoff[L];
-            for (int n = tid; n < N; n += kTrainThreads) {
-                float sb = 0.f;
-                for (int r = 0; r < nr; ++r) sb += delta[r * N + n];
-                atomicAdd(gb + n, sb);
-                for (int k = 0; k < K; ++k) {
-                    float s = 0.f;
-                    for (int r = 0; r < nr; ++r) s = fmaf(delta[r * N + n], a[r * K + k], s);
-                    atomicAdd(gW + (size_t)n * K + k, s);
-                }
+            const int K = net.dims[L], ni = (K + 31) / 32;
+            if (ni > 5) {
+                for (int i = 0; i < ni; i += 4) train_weights<4>(net, t, grad, L, 32 * i);
+            } else if (ni == 5) train_weights<5>(net, t, grad, L, 0);
+            else if (ni == 4) train_weights<4>(net, t, grad, L, 0);
+            else if (ni == 3) train_weights<3>(net, t, grad, L, 0);
+            else train_weights<2>(net, t, grad, L, 0);
+            train_bias(net, t, grad, L);
+            if (L == 0) break;
+            const int nc = train_columns(K, t.ncg), k0 = t.cg * nc;
+            const bool mine = t.on && k0 < K;
+            float4 d[8];
+            if (mine) {
+                if (nc == 8) {
+                    train_deltas<4>(net, t, w, L, k0, d);
+                    if (k0 + 4 < K) train_deltas<4>(net, t, w, L, k0 + 4, d + 4);
+                } else if (nc == 5) train_deltas<5>(net, t, w, L, k0, d);
+                else if (nc == 4) train_deltas<4>(net, t, w, L, k0, d);
+                else if (nc == 3) train_deltas<3>(net, t, w, L, k0, d);
+                else if (nc == 2) train_deltas<2>(net, t, w, L, k0, d);
+                else train_deltas<1>(net, t, w, L, k0, d);
             }
-            if (L > 0) {
-                // delta_{L-1}[r][k] = sum_n W[n][k] delta_L[r][n] * act'(z_{L-1}[r][k])
-                float *dprev = pre + net.aoff[L];
-                for (int k = tid; k < K; k += kTrainThreads) {
-                    float s[kTrainRows];
+            __syncthreads();  // every thread has read layer L's activations (its weight gradient)
+            if (mine) {
 #pragma unroll
-                    for (int r = 0; r < kTrainRows; ++r) s[r] = 0.f;
-                    for (int n = 0; n < N; ++n) {
-                        float wv = __ldg(W + (size_t)n * K + k);
-#pragma unroll
-                        for (int r = 0; r < kTrainRows; ++r) s[r] = fmaf(wv, delta[r * N + n], s[r]);
-                    }
-#pragma unroll
-                    for (int r = 0; r < kTrainRows; ++r) s[r] *= act_df(net.act, dprev[r * K + k]);
-#pragma unroll
-                    for (int r = 0; r < kTrainRows; ++r) dprev[r * K + k] = s[r];
+                for (int c = 0; c < 8; ++c) {
+                    // d[c] is the delta of column train_first(s0, ..) + c of its group
+                    const int s0 = nc == 8 && c >= 4 ? k0 + 4 : k0;
+                    const int k = nc == 8 ? train_first(s0, 4, K) + (c & 3) : train_first(s0, nc, K) + c;
+                    if (c < nc && s0 < K && k >= s0) train_store_delta(net, t, L, k, d[c]);
                 }
             }
             __syncthreads();
         }
+        __syncthreads();
     }
 }
 
@@ -141,23 +387,37 @@ static amlp_status launch_grad(const float *d_g, const float *d_y, const float *
     net.n_layers = mlp->n_layers;
     net.act = mlp->act;
     long long off = 0;
-    int aoff = 0;
+    int feat = 0;
     for (int k = 0; k <= mlp->n_layers; ++k) {
         net.dims[k] = mlp->dims[k];
         if (mlp->dims[k] > kTrainMaxWidth) return AMLP_ERR_UNSUPPORTED;
-        net.aoff[k] = aoff;
-        aoff += kTrainRows * mlp->dims[k];
+        net.feat[k] = feat;
+        feat += mlp->dims[k];
     }
+    if (feat > 880) return AMLP_ERR_UNSUPPORTED;  // the nets taken: layer widths, D and 1 included, adding up to 880
+    if (mlp->act == AMLP_ACT_SILU)
+        for (int k = 1; k < mlp->n_layers; ++k) {
+            net.zfeat[k] = feat;
+            feat += mlp->dims[k];
+        }
     for (int k = 0; k < mlp->n_layers; ++k) {
         net.woff[k] = off;
         off += (long long)mlp->dims[k + 1] * mlp->dims[k] + mlp->dims[k + 1];
     }
-    net.total = aoff;
-    size_t smem = (size_t)2 * aoff * sizeof(float);
-    if (smem > 220 * 1024) return AMLP_ERR_UNSUPPORTED;
+    // Rows per tile: as many as the shared memory holds, at most 64, then the fewest
+    // (a multiple of 4) with which the tiles make as few rounds of the SMs
+    int rg = kTrainMaxRows / 4;
+    while (rg > 1 && (size_t)feat * train_ld(rg) * sizeof(float) > kTrainSmem) --rg;
+    const long long rounds = (rows + (long long)kNumSM * 4 * rg - 1) / ((long long)kNumSM * 4 * rg);
+    const long long per = (rows + kNumSM * rounds - 1) / (kNumSM * rounds);
+    rg = (int)std::min<long long>(rg, std::max<long long>(1, (per + 3) / 4));
+    net.rg = rg;
+    net.ld = train_ld(rg);
+    const size_t smem = (size_t)feat * net.ld * sizeof(float);
+    if (smem > kTrainSmem) return AMLP_ERR_UNSUPPORTED;
     AMLP_CHECK_CUDA(cudaFuncSetAttribute(k_mlp_loss_grad, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    long long tiles = (rows + kTrainRows - 1) / kTrainRows;
-    int grid = (int)std::min<long long>(tiles, 4LL * kNumSM);
+    const long long tiles = (rows + 4 * rg - 1) / (4 * rg);
+    const int grid = (int)std::min<long long>(tiles, kNumSM);
     k_mlp_loss_grad<<<grid, kTrainThreads, smem, as_stream(stream)>>>(d_g, d_y, d_dy, rows, net, mlp->d_w, d_grad,
                                                                       d_dy ? nullptr : d_loss);
     return check_launch();
