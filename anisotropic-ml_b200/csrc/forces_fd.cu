@@ -296,74 +296,137 @@ __global__ void __launch_bounds__(kMlpRows) k_mlp(const float *g, long long rows
 // Register-tiled FP32 net for widths up to 160 (the reference's 150-wide models
 // on its own finite-difference data flow): tiles of 128 rows, 512 threads (four
 // warps per scheduler, which the shared memory of one tile allows). The
-// activations are feature-major in one shared-memory buffer, XT[k][col] (row
-// stride kTLd), with the tile's rows permuted so that thread rg's eight rows
-// sit at columns 4 rg .. 4 rg + 3 and 64 + 4 rg .. + 3: a quarter warp's
-// 16-byte loads cover 128 contiguous bytes. Each layer's weights are staged
-// k-major, WT[k][n] (row stride kTWs), by cp.async in blocks of 8 k x 4 n per
-// warp instruction (four 32-byte global segments, 32 different banks), so that
-// every copy of a thread is in flight at once; the next layer's copies run
-// while a layer's outputs are written. Thread t owns rows rg = t % 16 and, for
-// a 160-wide layer, columns 4 cg .. 4 cg + 3 and 128 + cg (cg = t / 16): per k
-// two 16-byte activation loads and two weight loads (16 and 4 bytes) feed 40
-// multiply-adds, the next k's operands loading while this k's multiply-adds
-// issue. Narrower layers take columns cg, cg + 32, ... below npad. The outputs
-// stay in registers until every thread has read the layer's inputs, then
-// overwrite them. Each hidden output is bias + sum_k x_k w_k in ascending k, one
-// rounding per multiply-add; the energy (the one-column output layer) is the
-// bias plus the 32 column groups' partial sums over k = cg, cg + 32, ...
+// activations are feature-major in one shared-memory buffer, XT[k][row] (row
+// stride kTLd). A lane owns four rows and a warp npad / 16 consecutive columns, up
+// to ten, so that the weights of a warp are the same for its lanes. Per two k, two
+// 16-byte activation loads and five 16-byte loads that broadcast (two columns' weights
+// of two k) feed 80 multiply-adds, issued as 40 pairs of columns, the next two k's
+// operands loading meanwhile. (A warp of 16 x 2 lanes with 8 rows x 5 columns each
+// took half as many again shared-memory wavefronts, 70 % of the SM's rate.)
+// Each warp stages its own columns' weights, WT[pair of columns][k][2], by cp.async
+// with the lanes along k: one 128-byte line of a row of W per instruction (a k-major
+// layout took four, and a quarter of the kernel's time). Two parts: k < kTSplit of
+// the next layer is copied while this layer's second part is multiplied (its first
+// part is free then), the rest while the outputs are written and the next
+// layer's first part is multiplied. Columns past the last are neither copied nor
+// used. The outputs stay in registers until every thread has read the layer's
+// inputs, then overwrite them. Each hidden output is bias + sum_k x_k w_k in
+// ascending k, one rounding per multiply-add; the energy (the one-column output
+// layer) is the bias plus the partial sums of 32 groups of threads over k = cg,
+// cg + 32, ... th_C104, 65,536 bodies (1.95 M rows): 7.80 -> 6.40 ms,
+// of which the products take about four fifths at 0.8 of the multiply-add rate.
 constexpr int kTRows = 128, kTThreads = 512, kTMaxW = 160, kTGroups = kTThreads / 16;
-constexpr int kTMaxCw = kTMaxW / kTGroups;  // outputs per row and thread: 5
-constexpr int kTLd = kTRows + 4;  // activation row stride (16-byte aligned rows)
-constexpr int kTWs = kTMaxW + 4;  // weight row stride: 16-byte aligned rows, 4 (mod 32) for the staging banks
-constexpr int kTRowsK = kTMaxW + 2;  // rows of XT and WT: K <= 160 plus the two that a prefetch may read past K
-__host__ __device__ constexpr int tiled_col(int r) { return ((r >> 2) & 1) * (kTRows / 2) + (r >> 3) * 4 + (r & 3); }
+constexpr int kTWarps = kTThreads / 32;
+constexpr int kTMaxP = kTMaxW / kTWarps / 2;  // pairs of columns per thread: 5
+constexpr int kTLd = kTRows + 4;  // activation row stride (16-byte aligned rows, 4 (mod 32) for the staging banks)
+constexpr int kTWp = 2 * kTMaxW + 4;  // floats per pair of columns
+constexpr int kTSplit = 96;           // k of a layer's first part (a multiple of 32)
+constexpr size_t kTSmem = sizeof(float) * ((size_t)kTMaxW * kTLd + (size_t)kTWarps * kTMaxP * kTWp + kTMaxW);
 
 // Asynchronous 4-byte global -> shared copy (cp.async, no register staging).
 __device__ __forceinline__ void cp_async4(float *dst, const float *src) {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src)
                  : "memory");
 }
-__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
-
-// Layer L's weights, k-major with zero columns up to npad, and its bias into
-// WT and Bs, in blocks of 8 k x 4 n per warp instruction. Copies in flight
-// until cp_async_wait_all.
-__device__ __forceinline__ void stage_layer(const MlpDesc &m, const float *w, int L, float *WT, float *Bs) {
-    const int K = m.dims[L], N = m.dims[L + 1], npad = (N + 15) / 16 * 16;
-    const float *W = w + m.woff[L], *b = W + (size_t)N * K;
-    const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
-    // warp w takes the column blocks w, w + 16, ... and walks each down k with
-    // two pointer increments per copy (no index division)
-    for (int nbi = warp; 4 * nbi < npad; nbi += kTThreads / 32) {
-        const int n = 4 * nbi + (lane & 3);
-        int k = lane >> 2;
-        float *dst = WT + k * kTWs + n;
-        if (n < N) {
-            const float *src = W + (size_t)n * K + k;
-            for (; k < K; k += 8, src += 8, dst += 8 * kTWs) cp_async4(dst, src);
-        } else {
-            for (; k < K; k += 8, dst += 8 * kTWs) *dst = 0.f;
-        }
-    }
-    for (int n = t; n < npad; n += kTThreads) {
-        if (n < N) cp_async4(Bs + n, b + n);
-        else Bs[n] = 0.f;
-    }
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+// Waits until at most N of this thread's groups of copies are in flight.
+template <int N>
+__device__ __forceinline__ void cp_async_wait() {
+    asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
 
-// Column of output c of thread group cg: a 160-wide layer (4 contiguous, then
-// one of the last 32), or a narrower one (cg + 32 c; beyond npad unused).
-__device__ __forceinline__ int wide_col(int cg, int c) { return c < 4 ? 4 * cg + c : 128 + cg; }
-__device__ __forceinline__ int narrow_col(int cg, int c) { return cg + kTGroups * c; }
+// Columns per warp of a layer of N outputs.
+__device__ __forceinline__ int tiled_cols(int N) { return (N + kTWarps - 1) / kTWarps; }
+
+// Weights k0 <= k < k1 (k0 a multiple of 32) of this warp's columns of layer L into
+// its part of WT, and with the first ones the layer's bias into Bs. One group of
+// copies, in flight until cp_async_wait.
+__device__ __forceinline__ void stage_weights(const MlpDesc &m, const float *w, int L, int k0, int k1, float *WT,
+                                              float *Bs) {
+    const int K = m.dims[L], N = m.dims[L + 1], end = min(K, k1), ncol = tiled_cols(N);
+    const float *W = w + m.woff[L], *b = W + (size_t)N * K;
+    const int t = threadIdx.x, lane = t & 31, n0 = (t >> 5) * ncol;
+    const float *src = W + (size_t)n0 * K + k0 + lane;
+    float *dst = WT + (t >> 5) * ((ncol + 1) / 2) * kTWp + 2 * (k0 + lane);
+    for (int j = 0; j < ncol && n0 + j < N; ++j, src += K) {
+        float *d = dst + (j >> 1) * kTWp + (j & 1);
+#pragma unroll
+        for (int i = 0; i < (kTMaxW + 31) / 32; ++i)
+            if (k0 + 32 * i + lane < end) cp_async4(d + 64 * i, src + 32 * i);
+    }
+    if (k0 == 0)
+        for (int n = t; n < N; n += kTThreads) cp_async4(Bs + n, b + n);
+    cp_async_commit();
+}
+
+// acc[i][c] (row i of the lane's four, columns 2 c and 2 c + 1 of the warp's) +=
+// sum over `count` k of x_k w_k, two k at a time; two operand sets alternate so
+// that the next two k are loading while these two's multiply-adds issue. x and w
+// point at the lane's and the warp's elements of the first k (w 16-byte aligned).
+template <int NP>
+__device__ __forceinline__ void tiled_product(float2 (&acc)[4][kTMaxP], const float *x, const float *w, int count) {
+    struct Ops {
+        float4 x0, x1, w[NP];
+    };
+    auto load = [&](int u) {
+        Ops o;
+        o.x0 = *reinterpret_cast<const float4 *>(x + u * kTLd);
+        o.x1 = *reinterpret_cast<const float4 *>(x + (u + 1) * kTLd);
+#pragma unroll
+        for (int c = 0; c < NP; ++c) o.w[c] = *reinterpret_cast<const float4 *>(w + c * kTWp + 2 * u);
+        return o;
+    };
+    auto mul1 = [&](const float4 &xv, const float2 (&wv)[NP]) {
+        const float xs[4] = {xv.x, xv.y, xv.z, xv.w};
+        // columns outside: a pair's four rows in a row (6.40 ms; rows outside 6.55, and with
+        // one fma of each five pairs as two scalar ones, 6.54)
+#pragma unroll
+        for (int c = 0; c < NP; ++c)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) acc[i][c] = fma2(make_float2(xs[i], xs[i]), wv[c], acc[i][c]);
+    };
+    auto mul = [&](const Ops &o) {
+        float2 w0[NP], w1[NP];
+#pragma unroll
+        for (int c = 0; c < NP; ++c)
+            w0[c] = make_float2(o.w[c].x, o.w[c].y), w1[c] = make_float2(o.w[c].z, o.w[c].w);
+        mul1(o.x0, w0);
+        mul1(o.x1, w1);
+    };
+    int pairs = count >> 1;
+    if (pairs > 0) {
+        Ops a = load(0);
+        for (; pairs > 2; pairs -= 2, x += 4 * kTLd, w += 8) {
+            const Ops b = load(2);
+            mul(a);
+            a = load(4);
+            mul(b);
+        }
+        if (pairs == 2) {
+            const Ops b = load(2);
+            mul(a);
+            mul(b);
+        } else {
+            mul(a);
+        }
+        x += 2 * pairs * kTLd;
+        w += 4 * pairs;
+    }
+    if (count & 1) {
+        float2 wv[NP];
+#pragma unroll
+        for (int c = 0; c < NP; ++c) wv[c] = *reinterpret_cast<const float2 *>(w + c * kTWp);
+        mul1(*reinterpret_cast<const float4 *>(x), wv);
+    }
+}
 
 __global__ void __launch_bounds__(kTThreads) k_mlp_tiled(const float *g, long long rows, MlpDesc m, const float *w,
                                                          float *e_out) {
     extern __shared__ __align__(16) float smem[];
-    float *XT = smem;                  // kTRowsK x kTLd
-    float *WT = XT + kTRowsK * kTLd;   // kTRowsK x kTWs
-    float *Bs = WT + kTRowsK * kTWs;   // kTMaxW
-    const int t = threadIdx.x, rg = t & 15, cg = t >> 4;
+    float *XT = smem;                // kTMaxW x kTLd
+    float *WT = XT + kTMaxW * kTLd;  // kTWarps x kTMaxP x kTWp
+    float *Bs = WT + kTWarps * kTMaxP * kTWp;  // kTMaxW
+    const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
     for (long long r0 = (long long)blockIdx.x * kTRows; r0 < rows; r0 += (long long)gridDim.x * kTRows) {
         const int D = m.dims[0];
         const int nr = (int)min((long long)kTRows, rows - r0);
@@ -371,10 +434,10 @@ __global__ void __launch_bounds__(kTThreads) k_mlp_tiled(const float *g, long lo
         // the tile's g rows, a warp instruction per 4 rows x 8 columns (four 32-byte
         // global segments; columns 4 apart in XT, 32 different banks), walked by
         // pointer increments
-        for (int rb = t >> 5; 4 * rb < kTRows; rb += kTThreads / 32) {
+        for (int rb = warp; 4 * rb < kTRows; rb += kTWarps) {
             const int rr = 4 * rb + (t & 3);
-            int d = (t & 31) >> 2;
-            float *dst = XT + d * kTLd + tiled_col(rr);
+            int d = lane >> 2;
+            float *dst = XT + d * kTLd + rr;
             if (rr < nr) {
                 const float *src = g + (r0 + rr) * D + d;
                 for (; d < D; d += 8, src += 8, dst += 8 * kTLd) cp_async4(dst, src);
@@ -382,26 +445,27 @@ __global__ void __launch_bounds__(kTThreads) k_mlp_tiled(const float *g, long lo
                 for (; d < D; d += 8, dst += 8 * kTLd) *dst = 0.f;
             }
         }
-        stage_layer(m, w, 0, WT, Bs);
-        cp_async_wait_all();
-        __syncthreads();
+        stage_weights(m, w, 0, 0, kTSplit, WT, Bs);
+        stage_weights(m, w, 0, kTSplit, kTMaxW, WT, Bs);
         for (int L = 0; L < m.n_layers; ++L) {
-            const int K = m.dims[L], N = m.dims[L + 1];
-            const int npad = (N + 15) / 16 * 16;
-            const bool last = L == m.n_layers - 1, wide = npad == kTMaxW;
-            const float *xk = XT + 4 * rg;
-            if (last) {
-                // the output layer (one column, N = 1): the 32 column groups split k (group
-                // cg sums k = cg, cg + 32, ... in ascending order over its 8 rows), the
+            const int K = m.dims[L], N = m.dims[L + 1], ks = min(K, kTSplit);
+            cp_async_wait<1>();  // this layer's first part (and the tile's inputs)
+            __syncthreads();
+            if (L == m.n_layers - 1) {
+                // the output layer (one column, N = 1): 32 groups of 16 threads split k (group
+                // cg sums k = cg, cg + 32, ... in ascending order, 8 rows per thread), the
                 // partial sums meet in the activation buffer and add up in group order
                 // after the bias
+                cp_async_wait<0>();
+                __syncthreads();
+                const int rg = t & 15, cg = t >> 4;
                 float part[8];
 #pragma unroll
                 for (int i = 0; i < 8; ++i) part[i] = 0.f;
                 for (int k = cg; k < K; k += kTGroups) {
-                    const float4 x0 = *reinterpret_cast<const float4 *>(xk + k * kTLd);
-                    const float4 x1 = *reinterpret_cast<const float4 *>(xk + k * kTLd + kTRows / 2);
-                    const float wv = WT[k * kTWs];
+                    const float4 x0 = *reinterpret_cast<const float4 *>(XT + k * kTLd + 8 * rg);
+                    const float4 x1 = *reinterpret_cast<const float4 *>(XT + k * kTLd + 8 * rg + 4);
+                    const float wv = WT[2 * k];
                     const float xs[8] = {x0.x, x0.y, x0.z, x0.w, x1.x, x1.y, x1.z, x1.w};
 #pragma unroll
                     for (int i = 0; i < 8; ++i) part[i] = fmaf(xs[i], wv, part[i]);
@@ -418,95 +482,49 @@ __global__ void __launch_bounds__(kTThreads) k_mlp_tiled(const float *g, long lo
                 }
                 break;
             }
-            const int ncol = wide ? kTMaxCw : (npad - cg + kTGroups - 1) / kTGroups;  // this thread's columns
-            float acc[8][kTMaxCw];
-            if (wide) {
+            const int ncol = tiled_cols(N), n0 = warp * ncol;
+            const float *xk = XT + 4 * lane, *wk = WT + warp * ((ncol + 1) / 2) * kTWp;
+            float2 acc[4][kTMaxP];
 #pragma unroll
-                for (int c = 0; c < kTMaxCw; ++c) {
-                    const float bc = Bs[wide_col(cg, c)];
+            for (int c = 0; c < kTMaxP; ++c) {
+                const float2 bc = make_float2(2 * c < ncol ? Bs[n0 + 2 * c] : 0.f,
+                                              2 * c + 1 < ncol ? Bs[n0 + 2 * c + 1] : 0.f);
 #pragma unroll
-                    for (int i = 0; i < 8; ++i) acc[i][c] = bc;
-                }
-                // operands of row k: x (8 rows) and w (5 columns); two sets alternate so
-                // that row k + 1 is loading while row k's 40 multiply-adds issue
-                struct Ops {
-                    float4 x0, x1, w0;
-                    float w1;
-                };
-                auto load = [&](const float *px, const float *pw) {
-                    Ops o;
-                    o.x0 = *reinterpret_cast<const float4 *>(px);
-                    o.x1 = *reinterpret_cast<const float4 *>(px + kTRows / 2);
-                    o.w0 = *reinterpret_cast<const float4 *>(pw + 4 * cg);
-                    o.w1 = pw[128 + cg];
-                    return o;
-                };
-                auto fma40 = [&](const Ops &o) {
-                    const float xs[8] = {o.x0.x, o.x0.y, o.x0.z, o.x0.w, o.x1.x, o.x1.y, o.x1.z, o.x1.w};
-                    const float ws[kTMaxCw] = {o.w0.x, o.w0.y, o.w0.z, o.w0.w, o.w1};
-#pragma unroll
-                    for (int c = 0; c < kTMaxCw; ++c)
-#pragma unroll
-                        for (int i = 0; i < 8; ++i) acc[i][c] = fmaf(xs[i], ws[c], acc[i][c]);
-                };
-                const float *px = xk, *pw = WT;
-                Ops a = load(px, pw);
-                for (int k = 0; k < K; k += 2, px += 2 * kTLd, pw += 2 * kTWs) {
-                    const Ops b = load(px + kTLd, pw + kTWs);  // row k + 1 (a padding row when k + 1 = K)
-                    fma40(a);
-                    if (k + 1 < K) {
-                        a = load(px + 2 * kTLd, pw + 2 * kTWs);  // row k + 2 (<= K + 1)
-                        fma40(b);
-                    }
-                }
-            } else if (ncol == 1) {  // one column (a hidden layer of width 16 or less: column cg < 16)
-#pragma unroll
-                for (int i = 0; i < 8; ++i) acc[i][0] = Bs[cg];
-                const float *px = xk, *pw = WT + cg;
-                for (int k = 0; k < K; ++k, px += kTLd, pw += kTWs) {
-                    const float4 x0 = *reinterpret_cast<const float4 *>(px);
-                    const float4 x1 = *reinterpret_cast<const float4 *>(px + kTRows / 2);
-                    const float wv = *pw;
-                    const float xs[8] = {x0.x, x0.y, x0.z, x0.w, x1.x, x1.y, x1.z, x1.w};
-#pragma unroll
-                    for (int i = 0; i < 8; ++i) acc[i][0] = fmaf(xs[i], wv, acc[i][0]);
-                }
-            } else if (ncol > 1) {
-#pragma unroll
-                for (int c = 0; c < kTMaxCw; ++c) {
-                    const float bc = c < ncol ? Bs[narrow_col(cg, c)] : 0.f;
-#pragma unroll
-                    for (int i = 0; i < 8; ++i) acc[i][c] = bc;
-                }
-                for (int k = 0; k < K; ++k) {
-                    const float4 x0 = *reinterpret_cast<const float4 *>(xk + k * kTLd);
-                    const float4 x1 = *reinterpret_cast<const float4 *>(xk + k * kTLd + kTRows / 2);
-                    const float xs[8] = {x0.x, x0.y, x0.z, x0.w, x1.x, x1.y, x1.z, x1.w};
-#pragma unroll
-                    for (int c = 0; c < kTMaxCw; ++c) {
-                        if (c < ncol) {
-                            const float wv = WT[k * kTWs + narrow_col(cg, c)];
-#pragma unroll
-                            for (int i = 0; i < 8; ++i) acc[i][c] = fmaf(xs[i], wv, acc[i][c]);
-                        }
-                    }
-                }
+                for (int i = 0; i < 4; ++i) acc[i][c] = bc;
             }
+            // (an odd last column's partner holds whatever the buffer held: its sums are not stored)
+            auto product = [&](int k0, int k1) {
+                const float *x = xk + k0 * kTLd, *wp = wk + 2 * k0;
+                switch ((ncol + 1) / 2) {
+                    case 1: tiled_product<1>(acc, x, wp, k1 - k0); break;
+                    case 2: tiled_product<2>(acc, x, wp, k1 - k0); break;
+                    case 3: tiled_product<3>(acc, x, wp, k1 - k0); break;
+                    case 4: tiled_product<4>(acc, x, wp, k1 - k0); break;
+                    default: tiled_product<5>(acc, x, wp, k1 - k0); break;
+                }
+            };
+            product(0, ks);
+            cp_async_wait<0>();  // this layer's second part
+            __syncthreads();     // and every thread has read its first part and the bias
+            stage_weights(m, w, L + 1, 0, kTSplit, WT, Bs);
+            product(ks, K);
             __syncthreads();  // every thread has read this layer's inputs and weights
-            stage_layer(m, w, L + 1, WT, Bs);  // in flight while the outputs are written
+            stage_weights(m, w, L + 1, kTSplit, kTMaxW, WT, Bs);
+            auto write = [&](auto act) {
 #pragma unroll
-            for (int c = 0; c < kTMaxCw; ++c) {
-                if (c < ncol) {
-                    float o[8];
+                for (int c = 0; c < 2 * kTMaxP; ++c) {
+                    if (c < ncol && n0 + c < N) {
+                        float o[4];
 #pragma unroll
-                    for (int i = 0; i < 8; ++i) o[i] = act_f(m.act, acc[i][c]);
-                    float *yp = XT + (wide ? wide_col(cg, c) : narrow_col(cg, c)) * kTLd + 4 * rg;
-                    *reinterpret_cast<float4 *>(yp) = make_float4(o[0], o[1], o[2], o[3]);
-                    *reinterpret_cast<float4 *>(yp + kTRows / 2) = make_float4(o[4], o[5], o[6], o[7]);
+                        for (int i = 0; i < 4; ++i) o[i] = act(c & 1 ? acc[i][c >> 1].y : acc[i][c >> 1].x);
+                        *reinterpret_cast<float4 *>(XT + (n0 + c) * kTLd + 4 * lane) =
+                            make_float4(o[0], o[1], o[2], o[3]);
+                    }
                 }
-            }
-            cp_async_wait_all();
-            __syncthreads();
+            };
+            if (m.act == AMLP_ACT_RELU) write([](float z) { return act_f(AMLP_ACT_RELU, z); });
+            else if (m.act == AMLP_ACT_TANH) write([](float z) { return act_f(AMLP_ACT_TANH, z); });
+            else write([](float z) { return act_f(AMLP_ACT_SILU, z); });
         }
     }
 }
@@ -882,11 +900,10 @@ extern "C" amlp_status amlp_mlp_energy(const float *d_g, long long rows, const a
         off += (long long)mlp->dims[k + 1] * mlp->dims[k] + mlp->dims[k + 1];
     }
     if (amax <= kTMaxW) {  // the register-tiled kernel
-        size_t smem = sizeof(float) * ((size_t)kTRowsK * kTLd + (size_t)kTRowsK * kTWs + kTMaxW);
-        if ((st = set_smem(k_mlp_tiled, smem))) return st;
+        if ((st = set_smem(k_mlp_tiled, kTSmem))) return st;
         long long tiles = (rows + kTRows - 1) / kTRows;
-        int grid = (int)std::min<long long>(tiles, kNumSM);  // one CTA per SM (188 KB of shared memory)
-        k_mlp_tiled<<<grid, kTThreads, smem, as_stream(stream)>>>(d_g, rows, m, mlp->d_w, d_e);
+        int grid = (int)std::min<long long>(tiles, kNumSM);  // one CTA per SM (206 KB of shared memory)
+        k_mlp_tiled<<<grid, kTThreads, kTSmem, as_stream(stream)>>>(d_g, rows, m, mlp->d_w, d_e);
         return check_launch();
     }
     size_t smem = 2 * sizeof(float) * (size_t)amax * kMlpRows;

@@ -1,8 +1,10 @@
 """The FP32 net kernels at the edges of their tiles, against FP64.
 
-k_mlp_loss_grad (weight gradients) splits rows and layer widths into register
-tiles: row counts around its tiles, widths to 256 and odd ones. Tolerance: 1e-5
-(norm) of the gradient and of the loss, the FP32 contract of the entry point.
+k_mlp_tiled (energies) and k_mlp_loss_grad (weight gradients) split rows, layer
+widths and the sum over inputs into register tiles and staged parts: row counts
+around their tiles, widths around 16, 80, 128 and 160 (256 for the gradient) and
+odd ones. Tolerances: 1e-5 of the largest energy, 1e-5 (norm) for a gradient,
+the FP32 contract of the two entry points.
 """
 import ctypes
 
@@ -27,6 +29,20 @@ def _net64(g, layers, act):
         if k + 1 < len(layers):
             g = ACTS[act](g)
     return g[:, 0]
+
+
+@pytest.mark.parametrize("rows", [1, 127, 128, 129, 300])
+@pytest.mark.parametrize("dims,act", [((47, 150, 150, 1), "relu"), ((121, 160, 144, 1), "tanh"),
+                                      ((47, 128, 79, 81, 1), "silu"), ((80, 16, 17, 1), "tanh"), ((160, 1), "relu"),
+                                      ((3, 1, 112, 113, 1), "silu")])
+def test_tiled_energies(dims, act, rows):
+    import gpu_helpers as H
+    layers = _layers(dims, 3)
+    g = np.random.default_rng(4).normal(0, 1, (rows, dims[0])).astype(np.float32)
+    e = H.mlp_energy(layers, act, g)
+    ref = _net64(torch.tensor(g).double(), [(torch.tensor(W).double(), torch.tensor(b).double()) for W, b in layers],
+                 act).numpy()
+    assert np.abs(e - ref).max() <= 1e-5 * max(1.0, np.abs(ref).max())
 
 
 @pytest.mark.parametrize("rows", [1, 3, 64, 65, 593, 9473])
