@@ -138,19 +138,20 @@ __device__ __forceinline__ void nep_descriptor(const PointFn &pt, int Nd, float 
         if (!((pass_mask >> pass) & 1u)) continue;  // uniform over the warp
         constexpr int KC = Cfg::KC;
         const int k0 = pass * KC;
-        float A[Cfg::NA][KC];
+        static_assert(KC % 2 == 0 && Cfg::K % KC == 0, "whole pairs of harmonics per pass");
+        float2 A[Cfg::NA][KC / 2];  // pairs of harmonics
         float R[Cfg::NR];
 #pragma unroll
         for (int n = 0; n < Cfg::NA; ++n)
 #pragma unroll
-            for (int kk = 0; kk < KC; ++kk) A[n][kk] = 0.f;
+            for (int k2 = 0; k2 < KC / 2; ++k2) A[n][k2] = make_float2(0.f, 0.f);
 #pragma unroll
         for (int n = 0; n < Cfg::NR; ++n) R[n] = 0.f;
         for (int a = 0; a < Nd; ++a) {
             float3 p = pt(a);
             float rx = p.x - cx, ry = p.y - cy, rz = p.z - cz;
             float d2 = fmaf(rx, rx, fmaf(ry, ry, rz * rz));
-            float inv_d = rsqrtf(d2);
+            float inv_d = rsqrt_ftz(d2);
             float d = d2 * inv_d;
             float f[Cfg::NR];
             radial_basis<Cfg::NR>(d, inv_rc, f);
@@ -163,8 +164,8 @@ __device__ __forceinline__ void nep_descriptor(const PointFn &pt, int Nd, float 
 #pragma unroll
             for (int n = 0; n < Cfg::NA; ++n)
 #pragma unroll
-                for (int kk = 0; kk < KC; ++kk)
-                    if (k0 + kk < Cfg::K) A[n][kk] = fmaf(f[n], Y[k0 + kk], A[n][kk]);
+                for (int k2 = 0; k2 < KC / 2; ++k2)
+                    A[n][k2] = fma2(make_float2(f[n], f[n]), make_float2(Y[k0 + 2 * k2], Y[k0 + 2 * k2 + 1]), A[n][k2]);
         }
         if (pass == 0) {
 #pragma unroll
@@ -180,8 +181,10 @@ __device__ __forceinline__ void nep_descriptor(const PointFn &pt, int Nd, float 
                 float *e = g + (Cfg::NR + n * Cfg::LMAX + l - 1) * gstride;
                 float s = *e;
 #pragma unroll
-                for (int kk = 0; kk < KC; ++kk)
-                    if (k0 + kk < Cfg::K && sh_l_of(k0 + kk) == l) s = fmaf(A[n][kk], A[n][kk], s);
+                for (int kk = 0; kk < KC; ++kk) {
+                    const float a = kk & 1 ? A[n][kk >> 1].y : A[n][kk >> 1].x;
+                    if (sh_l_of(k0 + kk) == l) s = fmaf(a, a, s);
+                }
                 *e = s;
             }
         }

@@ -140,7 +140,7 @@ __device__ __forceinline__ void build_cloud(float4 *S, const float *pos, const f
         if (a >= npts) r.x += t.x, r.y += t.y, r.z += t.z;
         r.x -= cen.x, r.y -= cen.y, r.z -= cen.z;
         const float d2 = fmaf(r.x, r.x, fmaf(r.y, r.y, r.z * r.z));
-        const float inv_d = rsqrtf(d2);
+        const float inv_d = rsqrt_ftz(d2);
         S[a * kThreads] = make_float4(r.x * inv_d, r.y * inv_d, r.z * inv_d, d2 * inv_d);
     }
 }
@@ -164,12 +164,14 @@ __global__ void __launch_bounds__(kThreads) k_desc_direct_fwd(const float *pos, 
         float3 t, cen;
         float mi[9], mj[9];
         build_cloud(S, pos, quat, L, pairs[2 * q], pairs[2 * q + 1], pts, npts, psum, t, cen, mi, mj);
-        float acc[NA][LM], rad[NR], dia[NA];
+        static_assert(LM % 2 == 0, "whole pairs of degrees");
+        float2 acc[NA][LM / 2];  // pairs of degrees l
+        float rad[NR], dia[NA];
 #pragma unroll
         for (int n = 0; n < NA; ++n) {
             dia[n] = 0.f;
 #pragma unroll
-            for (int l = 0; l < LM; ++l) acc[n][l] = 0.f;
+            for (int l = 0; l < LM / 2; ++l) acc[n][l] = make_float2(0.f, 0.f);
         }
 #pragma unroll
         for (int n = 0; n < NR; ++n) rad[n] = 0.f;
@@ -195,7 +197,8 @@ __global__ void __launch_bounds__(kThreads) k_desc_direct_fwd(const float *pos, 
                 for (int n = 0; n < NA; ++n) {
                     const float ff = fa[n] * fb[n];
 #pragma unroll
-                    for (int l = 0; l < LM; ++l) acc[n][l] = fmaf(ff, Pl[l], acc[n][l]);
+                    for (int l = 0; l < LM / 2; ++l)
+                        acc[n][l] = fma2(make_float2(ff, ff), make_float2(Pl[2 * l], Pl[2 * l + 1]), acc[n][l]);
                 }
             }
         }
@@ -205,7 +208,7 @@ __global__ void __launch_bounds__(kThreads) k_desc_direct_fwd(const float *pos, 
             if (col < NR) return rad[col];
             if (col < D) {
                 const int n = (col - NR) / LM, l = (col - NR) % LM;
-                return fmaf(2.0f, acc[n][l], dia[n]);
+                return fmaf(2.0f, l & 1 ? acc[n][l >> 1].y : acc[n][l >> 1].x, dia[n]);
             }
             return 0.f;
         };

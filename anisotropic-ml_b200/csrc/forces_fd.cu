@@ -154,15 +154,17 @@ __device__ __forceinline__ void direct_row_descriptor(const VariantPoints &vp, i
         const float3 p = vp(a);
         const float rx = p.x - cx, ry = p.y - cy, rz = p.z - cz;
         const float d2 = fmaf(rx, rx, fmaf(ry, ry, rz * rz));
-        const float inv_d = rsqrtf(d2);
+        const float inv_d = rsqrt_ftz(d2);
         S[a * sstride] = make_float4(rx * inv_d, ry * inv_d, rz * inv_d, d2 * inv_d);
     }
-    float acc[NA][LM], rad[NR], dia[NA];
+    static_assert(LM % 2 == 0, "whole pairs of degrees");
+    float2 acc[NA][LM / 2];  // pairs of degrees l
+    float rad[NR], dia[NA];
 #pragma unroll
     for (int n = 0; n < NA; ++n) {
         dia[n] = 0.f;
 #pragma unroll
-        for (int l = 0; l < LM; ++l) acc[n][l] = 0.f;
+        for (int l = 0; l < LM / 2; ++l) acc[n][l] = make_float2(0.f, 0.f);
     }
 #pragma unroll
     for (int n = 0; n < NR; ++n) rad[n] = 0.f;
@@ -188,7 +190,8 @@ __device__ __forceinline__ void direct_row_descriptor(const VariantPoints &vp, i
             for (int n = 0; n < NA; ++n) {
                 const float ff = fa[n] * fb[n];
 #pragma unroll
-                for (int l = 0; l < LM; ++l) acc[n][l] = fmaf(ff, Pl[l], acc[n][l]);
+                for (int l = 0; l < LM / 2; ++l)
+                    acc[n][l] = fma2(make_float2(ff, ff), make_float2(Pl[2 * l], Pl[2 * l + 1]), acc[n][l]);
             }
         }
     }
@@ -197,7 +200,10 @@ __device__ __forceinline__ void direct_row_descriptor(const VariantPoints &vp, i
 #pragma unroll
     for (int n = 0; n < NA; ++n)
 #pragma unroll
-        for (int l = 0; l < LM; ++l) g[(NR + n * LM + l) * gstride] = fmaf(2.0f, acc[n][l], dia[n]);
+        for (int l = 0; l < LM / 2; ++l) {
+            g[(NR + n * LM + 2 * l) * gstride] = fmaf(2.0f, acc[n][l].x, dia[n]);
+            g[(NR + n * LM + 2 * l + 1) * gstride] = fmaf(2.0f, acc[n][l].y, dia[n]);
+        }
 }
 
 template <int NR, int NA, int LM>
@@ -588,7 +594,7 @@ static_assert(kFusedThreads % 128 == 0, "the fused kernel's warps are a multiple
 __host__ __device__ constexpr int act_col(int r) { return ((r >> 2) & 1) * (kRows / 2) + (r >> 3) * 4 + (r & 3); }
 
 // YT[n][r] = act(b[n] + sum_k XT[k][r] WT[k*npad + n]) for n < npad, rows in the
-// permuted layout above; 8x8 register tiles. The items are dealt to the SM's
+// permuted layout above; 8x8 register tiles, 32 pairs of rows per k. The items are dealt to the SM's
 // four schedulers (warp % 4) in four equal consecutive ranges, a quarter of the
 // work each (the block holds the same number of warps per scheduler); inside a
 // range the scheduler's warps take consecutive items.
@@ -601,12 +607,12 @@ __device__ __forceinline__ void tile_gemm(const float *XT, int K, const float *W
     for (int li = (warp >> 2) * 32 + (threadIdx.x & 31); li < per; li += per_sched) {
         const int it = base + li;
         const int rg = it % nrg, cg = it / nrg;
-        float acc[8][8];
+        float2 acc[4][8];  // rows 2 i, 2 i + 1
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
             float bj = b[cg * 8 + j];
 #pragma unroll
-            for (int i = 0; i < 8; ++i) acc[i][j] = bj;
+            for (int i = 0; i < 4; ++i) acc[i][j] = make_float2(bj, bj);
         }
         // operands of row k; two sets alternate so that row k + 1 loads while row k's 64
         // multiply-adds issue. The load of row K (past the last) reads the next area of
@@ -623,12 +629,13 @@ __device__ __forceinline__ void tile_gemm(const float *XT, int K, const float *W
             return o;
         };
         auto fma64 = [&](const Ops &o) {
-            const float xs[8] = {o.x0.x, o.x0.y, o.x0.z, o.x0.w, o.x1.x, o.x1.y, o.x1.z, o.x1.w};
+            const float2 xs[4] = {make_float2(o.x0.x, o.x0.y), make_float2(o.x0.z, o.x0.w),
+                                  make_float2(o.x1.x, o.x1.y), make_float2(o.x1.z, o.x1.w)};
             const float ws[8] = {o.w0.x, o.w0.y, o.w0.z, o.w0.w, o.w1.x, o.w1.y, o.w1.z, o.w1.w};
 #pragma unroll
-            for (int i = 0; i < 8; ++i)
+            for (int j = 0; j < 8; ++j)
 #pragma unroll
-                for (int j = 0; j < 8; ++j) acc[i][j] = fmaf(xs[i], ws[j], acc[i][j]);
+                for (int i = 0; i < 4; ++i) acc[i][j] = fma2(xs[i], make_float2(ws[j], ws[j]), acc[i][j]);
         };
         const float *xp = XT + rg * 4, *wp = WT + cg * 8;
         Ops a = load(xp, wp);
@@ -644,7 +651,7 @@ __device__ __forceinline__ void tile_gemm(const float *XT, int K, const float *W
         for (int j = 0; j < 8; ++j) {
             float o[8];
 #pragma unroll
-            for (int i = 0; i < 8; ++i) o[i] = act_f(act, acc[i][j]);
+            for (int i = 0; i < 4; ++i) o[2 * i] = act_f(act, acc[i][j].x), o[2 * i + 1] = act_f(act, acc[i][j].y);
             float *yp = YT + (cg * 8 + j) * kRows + rg * 4;
             *reinterpret_cast<float4 *>(yp) = make_float4(o[0], o[1], o[2], o[3]);
             *reinterpret_cast<float4 *>(yp + hoff) = make_float4(o[4], o[5], o[6], o[7]);
