@@ -526,23 +526,52 @@ __device__ __forceinline__ void mma3(uint32_t d_tmem, const char *a_hi, int K, c
     }
 }
 
-// Write 8 consecutive values of row p, columns c0..c0+7 into a K-major bf16
-// hi/lo tile of width K.
-// The splits are rounded two at a time (one packed conversion per pair, the
-// same round-to-nearest-even values as tc::split_bf16).
-__device__ __forceinline__ void store_split8(char *tile_hi, int K, int p, int c0, const float *v) {
-    uint32_t hi[4], lo[4];
+// bf16 hi and lo of 8 values, rounded two at a time (one packed conversion per
+// pair, the same round-to-nearest-even values as tc::split_bf16).
+__device__ __forceinline__ void split8(const float *v, uint4 &hi, uint4 &lo) {
+    uint32_t h[4], l[4];
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
         const __nv_bfloat162 h2 = __floats2bfloat162_rn(v[2 * k], v[2 * k + 1]);
         const float2 hf = __bfloat1622float2(h2);
         const __nv_bfloat162 l2 = __floats2bfloat162_rn(v[2 * k] - hf.x, v[2 * k + 1] - hf.y);
-        hi[k] = *reinterpret_cast<const uint32_t *>(&h2);
-        lo[k] = *reinterpret_cast<const uint32_t *>(&l2);
+        h[k] = *reinterpret_cast<const uint32_t *>(&h2);
+        l[k] = *reinterpret_cast<const uint32_t *>(&l2);
     }
-    uint32_t off = tc::kmajor_offset(p, c0, K);
-    *reinterpret_cast<uint4 *>(tile_hi + off) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
-    *reinterpret_cast<uint4 *>(tile_hi + kAP * K * 2 + off) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+    hi = make_uint4(h[0], h[1], h[2], h[3]);
+    lo = make_uint4(l[0], l[1], l[2], l[3]);
+}
+
+// Write 8 consecutive values of row p, columns c0..c0+7 into a K-major bf16
+// hi/lo tile of width K.
+__device__ __forceinline__ void store_split8(char *tile_hi, int K, int p, int c0, const float *v) {
+    uint4 hi, lo;
+    split8(v, hi, lo);
+    const uint32_t off = tc::kmajor_offset(p, c0, K);
+    *reinterpret_cast<uint4 *>(tile_hi + off) = hi;
+    *reinterpret_cast<uint4 *>(tile_hi + kAP * K * 2 + off) = lo;
+}
+
+// The weights of a layer (N x K, row-major) as a zero-padded Np x Kp K-major bf16
+// hi/lo operand: hi at `hi`, lo after it. Eight weights per thread and step
+// (independent loads, 16-byte stores), `first` of `stride` threads.
+// One weight per step, with a division and 2-byte stores each, took every block of
+// the fused kernel 6 us: 83.6 us a pass over 1,000 cubes, 77.5 us so.
+__device__ __forceinline__ void split_layer(const float *W, int N, int K, int Np, int Kp, char *hi, int first,
+                                            int stride) {
+    char *lo = hi + (size_t)Np * Kp * 2;
+    const int per_row = Kp / 8;
+    for (int c = first; c < Np * per_row; c += stride) {
+        const int n = c / per_row, k0 = 8 * (c - n * per_row);
+        float v[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) v[u] = n < N && k0 + u < K ? W[(size_t)n * K + k0 + u] : 0.f;
+        uint4 h, l;
+        split8(v, h, l);
+        const uint32_t off = tc::kmajor_offset(n, k0, Kp);
+        *reinterpret_cast<uint4 *>(hi + off) = h;
+        *reinterpret_cast<uint4 *>(lo + off) = l;
+    }
 }
 
 // Centroid of pair q's cloud into S.cen from its orientations and translation
@@ -788,17 +817,7 @@ __global__ void __launch_bounds__(kAThreads, 1) k_forces_adjoint(const float *po
     for (int L2 = 0; L2 < net.nh; ++L2) {
         const int K = net.dims[L2], N = net.dims[L2 + 1], Kp = net.kin[L2], Np = net.nout[L2];
         const float *W = w + net.woff[L2];
-        char *hi = S.wts + net.wsm_off[L2];
-        char *lo = hi + Np * Kp * 2;
-        for (int idx = tid; idx < Np * Kp; idx += kAThreads) {
-            int n = idx / Kp, k = idx - n * Kp;
-            float v = (n < N && k < K) ? W[(size_t)n * K + k] : 0.f;
-            __nv_bfloat16 a, b;
-            tc::split_bf16(v, a, b);
-            uint32_t o = tc::kmajor_offset(n, k, Kp);
-            *reinterpret_cast<__nv_bfloat16 *>(hi + o) = a;
-            *reinterpret_cast<__nv_bfloat16 *>(lo + o) = b;
-        }
+        split_layer(W, N, K, Np, Kp, S.wts + net.wsm_off[L2], tid, kAThreads);
         const float *b = W + (size_t)N * K;
         for (int n = tid; n < Np; n += kAThreads) S.par[net.bias_off[L2] + n] = n < N ? b[n] : 0.f;
     }
@@ -1172,17 +1191,8 @@ __global__ void __launch_bounds__(kDThreads, 2) k_adj_desc(const float *pos, con
 __global__ void k_split_weights(AdjNet net, const float *w, char *dst) {
     for (int L2 = 0; L2 < net.nh; ++L2) {
         const int K = net.dims[L2], N = net.dims[L2 + 1], Kp = net.kin[L2], Np = net.nout[L2];
-        const float *W = w + net.woff[L2];
-        char *hi = dst + net.wsm_off[L2], *lo = hi + (size_t)Np * Kp * 2;
-        for (int idx = blockIdx.x * blockDim.x + threadIdx.x; idx < Np * Kp; idx += gridDim.x * blockDim.x) {
-            int n = idx / Kp, k = idx - n * Kp;
-            float v = (n < N && k < K) ? W[(size_t)n * K + k] : 0.f;
-            __nv_bfloat16 a, bb;
-            tc::split_bf16(v, a, bb);
-            uint32_t o = tc::kmajor_offset(n, k, Kp);
-            *reinterpret_cast<__nv_bfloat16 *>(hi + o) = a;
-            *reinterpret_cast<__nv_bfloat16 *>(lo + o) = bb;
-        }
+        split_layer(w + net.woff[L2], N, K, Np, Kp, dst + net.wsm_off[L2], blockIdx.x * blockDim.x + threadIdx.x,
+                    gridDim.x * blockDim.x);
     }
 }
 
@@ -1691,7 +1701,7 @@ static amlp_status launch_adjoint_wide(const float *d_pos, const float *d_quat, 
                                 (const float *)nep->d_pts, npts, inv_rc, g_rows, grow)))
             return st;
         stage_mark(1, s);
-        k_split_weights<<<64, 256, 0, s>>>(net, mlp->d_w, wsplit);
+        k_split_weights<<<kNumSM, 128, 0, s>>>(net, mlp->d_w, wsplit);
         k_mlp_grad<<<kNumSM, kMThreads, net.smem, s>>>(g_rows, d_npairs, cap, net, mlp->d_w, wsplit, y_rows, dg_rows);
         stage_mark(2, s);
         if ((st = launch_direct(bwd, cap, npts, s, d_pos, d_quat, box, d_pairs, d_npairs, cap,
@@ -1724,7 +1734,7 @@ static amlp_status launch_adjoint_wide(const float *d_pos, const float *d_quat, 
                                              nep->en_min, rng, g_rows, kGRow, nullptr, nullptr, nullptr, clip, d_F,
                                              d_T, d_pe, d_rep, d_rp, a_rows);
     stage_mark(1, s);
-    k_split_weights<<<64, 256, 0, s>>>(net, mlp->d_w, wsplit);
+    k_split_weights<<<kNumSM, 128, 0, s>>>(net, mlp->d_w, wsplit);
     k_mlp_grad<<<kNumSM, kMThreads, smem_mlp, s>>>(g_rows, d_npairs, cap, net, mlp->d_w, wsplit, y_rows, dg_rows);
     stage_mark(2, s);
     bwd<<<2 * kNumSM, kDThreads, smem_desc, s>>>(d_pos, d_quat, box, d_pairs, d_npairs, cap, nep->d_pts, npts, inv_rc,
