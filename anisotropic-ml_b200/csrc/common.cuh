@@ -101,6 +101,28 @@ __device__ __forceinline__ float rsqrt_ftz(float x) {
     return r;
 }
 
+// 2^x and 1 / x by the hardware approximations, subnormals as 0 (without the scaling
+// around them that the general forms carry).
+__device__ __forceinline__ float exp2_ftz(float x) {
+    float r;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+__device__ __forceinline__ float rcp_ftz(float x) {
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+
+// Two sums in one instruction, each rounded as a + b.
+__device__ __forceinline__ float2 add2(float2 a, float2 b) {
+    float2 d;
+    asm("add.rn.f32x2 %0, %1, %2;"
+        : "=l"(reinterpret_cast<unsigned long long &>(d))
+        : "l"(reinterpret_cast<const unsigned long long &>(a)), "l"(reinterpret_cast<const unsigned long long &>(b)));
+    return d;
+}
+
 // True when the keys of the valid lanes never decrease from one lane to the
 // next, so that equal keys form contiguous runs and a segmented warp sum over
 // runs is exact. `ok` marks the valid lanes, a prefix of the warp. Pair lists

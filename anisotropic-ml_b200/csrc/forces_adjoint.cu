@@ -61,29 +61,50 @@ struct AdjNet {
     int wsm_total;                       // bytes of the weight area
     int bias_off[kMaxHiddenWide + 1];    // float offsets of b_k in the fp32 parameter area; last = w_last
     int par_total;
-    // k_mlp_grad only (set by wide_net): row strides of the g and dE/dg rows, widest
+    // the wide path's net kernels only (set by wide_net): row strides of the g and dE/dg rows, widest
     // hidden layer, TMEM columns of the product region, act'(z) as bits (ReLU),
     // shared-memory carve-up and whether the next tile's g rows are prefetched
     int g_ld, gp, wmax, zbw, relu_bits;
     int wbuf_off, par_off, eps_off, gbuf_off, prefetch_g, smem;
+    // k_mlp_pair: 0 not taken, 1 both operand tiles in shared memory, 2 the first in TMEM
+    int pair, pair_d, pair_tile, pair_wbuf, pair_par, pair_eps, pair_smem;
 };
 
 // Activation and its derivative from one exponential, for the tensor-core
 // epilogues (the net there is accurate to about 1e-5 relative, so the fast
 // exponential's few-ulp error does not show): tanh(z) = 1 - 2 / (1 + e^(2z)),
 // tanh' = 1 - tanh^2; silu(z) = z s, silu' = s (1 + z (1 - s)), s = 1 / (1 + e^-z).
-__device__ __forceinline__ void act_pair(int act, float z, float &f, float &df) {
-    if (act == AMLP_ACT_RELU) {
+// The exponential and the reciprocal flush subnormals: where one occurs it is added
+// to 1 or is a saturated derivative's factor, and every float gives the value that
+// the general forms give, at less than half of their instructions.
+template <int ACT>
+__device__ __forceinline__ void act_pair(float z, float &f, float &df) {
+    constexpr float kLog2e = 1.4426950408889634f;
+    if (ACT == AMLP_ACT_RELU) {
         f = fmaxf(z, 0.0f);
         df = z > 0.0f ? 1.0f : 0.0f;
-    } else if (act == AMLP_ACT_TANH) {
-        const float t = 1.0f - __fdividef(2.0f, 1.0f + __expf(2.0f * z));
+    } else if (ACT == AMLP_ACT_TANH) {
+        const float t = fmaf(-2.0f, rcp_ftz(1.0f + exp2_ftz(z * (2.0f * kLog2e))), 1.0f);
         f = t;
         df = fmaf(-t, t, 1.0f);
     } else {
-        const float sg = __fdividef(1.0f, 1.0f + __expf(-z));
+        const float sg = rcp_ftz(1.0f + exp2_ftz(-z * kLog2e));
         f = z * sg;
         df = sg * fmaf(z, 1.0f - sg, 1.0f);
+    }
+}
+
+// Eight of them, one branch on the activation.
+__device__ __forceinline__ void act8(int act, const float *z, float *f, float *df) {
+    if (act == AMLP_ACT_RELU) {
+#pragma unroll
+        for (int k = 0; k < 8; ++k) act_pair<AMLP_ACT_RELU>(z[k], f[k], df[k]);
+    } else if (act == AMLP_ACT_TANH) {
+#pragma unroll
+        for (int k = 0; k < 8; ++k) act_pair<AMLP_ACT_TANH>(z[k], f[k], df[k]);
+    } else {
+#pragma unroll
+        for (int k = 0; k < 8; ++k) act_pair<AMLP_ACT_SILU>(z[k], f[k], df[k]);
     }
 }
 
@@ -534,7 +555,8 @@ __device__ __forceinline__ void split8(const float *v, uint4 &hi, uint4 &lo) {
     for (int k = 0; k < 4; ++k) {
         const __nv_bfloat162 h2 = __floats2bfloat162_rn(v[2 * k], v[2 * k + 1]);
         const float2 hf = __bfloat1622float2(h2);
-        const __nv_bfloat162 l2 = __floats2bfloat162_rn(v[2 * k] - hf.x, v[2 * k + 1] - hf.y);
+        const float2 r = add2(make_float2(v[2 * k], v[2 * k + 1]), make_float2(-hf.x, -hf.y));
+        const __nv_bfloat162 l2 = __floats2bfloat162_rn(r.x, r.y);
         h[k] = *reinterpret_cast<const uint32_t *>(&h2);
         l[k] = *reinterpret_cast<const uint32_t *>(&l2);
     }
@@ -929,15 +951,13 @@ __global__ void __launch_bounds__(kAThreads, 1) k_forces_adjoint(const float *po
                             *reinterpret_cast<float4 *>(ww + 4) = *reinterpret_cast<const float4 *>(wl + c0 + 4);
                         }
 #pragma unroll
-                        for (int k = 0; k < 8; ++k) {
-                            float zz = z[8 * ch + k] + bb[k], fz, dfz;
-                            act_pair(net.act, zz, fz, dfz);
-                            if (last) {
-                                esum = fmaf(ww[k], fz, esum);
-                                v[k] = ww[k] * dfz;
-                            } else {
-                                v[k] = fz;
-                                dv[k] = dfz;
+                        for (int k = 0; k < 8; ++k) bb[k] += z[8 * ch + k];
+                        act8(net.act, bb, v, dv);
+                        if (last) {
+#pragma unroll
+                            for (int k = 0; k < 8; ++k) {
+                                esum = fmaf(ww[k], v[k], esum);
+                                v[k] = ww[k] * dv[k];
                             }
                         }
                         store_split8(dst, Np, p, c0, v);
@@ -1043,7 +1063,7 @@ __global__ void __launch_bounds__(kAThreads, 1) k_forces_adjoint(const float *po
 // CTA's shared memory. g, dE/dg and the net output go through a caller
 // workspace:
 //   k_adj_desc<..., false>  descriptor forward per pair -> g (P x 48 fp32);
-//   k_mlp_grad              net forward + backward on the tensor cores per row,
+//   k_mlp_pair, k_mlp_grad  net forward + backward on the tensor cores per row,
 //                           weights staged layer by layer -> y and dE/dg;
 //   k_adj_desc<..., true>   recomputes the per-pair sums, descriptor backward,
 //                           forces, torques, scatter.
@@ -1187,7 +1207,7 @@ __global__ void __launch_bounds__(kDThreads, 2) k_adj_desc(const float *pos, con
 
 // The hidden layers' weights split into bf16 hi/lo once per launch, in the
 // K-major layout of the shared-memory operand (per layer: hi, then lo), so that
-// k_mlp_grad loads a layer with one bulk copy.
+// the net kernels load a layer with one bulk copy.
 __global__ void k_split_weights(AdjNet net, const float *w, char *dst) {
     for (int L2 = 0; L2 < net.nh; ++L2) {
         const int K = net.dims[L2], N = net.dims[L2 + 1], Kp = net.kin[L2], Np = net.nout[L2];
@@ -1356,17 +1376,17 @@ __global__ void __launch_bounds__(kMThreads, 1) k_mlp_grad(const float *g_rows, 
                 }
                 uint32_t b8 = 0;
 #pragma unroll
-                for (int k = 0; k < 8; ++k) {
-                    float zz = z[k] + bb[k], fz, dfz;
-                    act_pair(net.act, zz, fz, dfz);
-                    if (last) {
-                        esum = fmaf(ww[k], fz, esum);
-                        v[k] = ww[k] * dfz;
-                    } else {
-                        v[k] = fz;
-                        dv[k] = dfz;
-                        b8 |= (dfz != 0.f ? 1u : 0u) << k;
+                for (int k = 0; k < 8; ++k) bb[k] += z[k];
+                act8(net.act, bb, v, dv);
+                if (last) {
+#pragma unroll
+                    for (int k = 0; k < 8; ++k) {
+                        esum = fmaf(ww[k], v[k], esum);
+                        v[k] = ww[k] * dv[k];
                     }
+                } else if (relu) {
+#pragma unroll
+                    for (int k = 0; k < 8; ++k) b8 |= (dv[k] != 0.f ? 1u : 0u) << k;
                 }
                 if (!last) bits |= (uint64_t)b8 << (8 * j);
                 store_split8(tile, Np, p, c0, v);  // the MMA that read the tile is complete
@@ -1451,6 +1471,394 @@ __global__ void __launch_bounds__(kMThreads, 1) k_mlp_grad(const float *g_rows, 
     if (warp == 0) {
         tc::fence_after();
         tc::tmem_dealloc(tmem, 512);
+    }
+}
+
+// The same net pass with two tiles in flight per CTA. k_mlp_grad runs a tile's products
+// and epilogues one after the other: of its 51 k cycles a tile (four 160-wide layers)
+// the tensor cores worked 20 k. Here two teams of eight warps each have a tile of their
+// own (operand tile, product region, mbarrier), so that one team's epilogue runs under
+// the other's product, and one copy of the running layer's weights serves both.
+//  - Warp 17 issues the products, team 0's then team 1's of each layer, when a team
+//    signals that its operand tile is written (ready) and the weights are there (wfull).
+//    All its lanes compute the descriptors, so that they stay in uniform registers:
+//    issued by a thread of the team under a divergent branch, between its scheduler's
+//    epilogues, the 30 MMAs of a 160-wide layer took 3.9 k cycles to issue and 2.4 k to run.
+//  - Warp 16 copies the next layer's weights when both products are complete (wfree).
+//  - A team without a tile (last round) is left out of the round.
+// Two 160-wide operand tiles and a layer's weights do not fit shared memory: with TMEM_A
+// the first team's operand tile is in TMEM (bf16 pairs, hi and lo), which ReLU leaves
+// room for (its derivatives are bits in registers). Smooth activations take this kernel
+// when both tiles fit shared memory and both teams' act'(z) fit TMEM; up to two 128-wide
+// hidden layers do. A product is the same sequence of MMAs as in k_mlp_grad. The
+// epilogues, two chunks of 8 columns a step with the activation known at compile time,
+// take 40 % of the issue slots and bound the kernel with the products' latency.
+// Measured against k_mlp_grad: 5,465 tiles of four 150-wide ReLU layers 960 -> 627 us
+// (tensor pipe busy 336 us), 5,715 tiles of two 128-wide silu layers 490 -> 364 us.
+constexpr int kPTeam = 256;
+constexpr int kPThreads = 2 * kPTeam + 64;
+
+__device__ __forceinline__ bool pair_sync_or(int team, bool v) {
+    uint32_t o;
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\t"
+        "setp.ne.u32 p, %1, 0;\n\t"
+        "barrier.cta.red.or.pred q, %2, %3, p;\n\t"
+        "selp.u32 %0, 1, 0, q;\n\t}\n"
+        : "=r"(o)
+        : "r"((uint32_t)v), "r"(1 + team), "n"(kPTeam)
+        : "memory");
+    return o != 0;
+}
+
+// mma3's sequence with the descriptors' steps added to their address fields (a shared-memory
+// address is below 2^18, so a field holds it) and, with a_tmem, A's hi and lo in TMEM.
+// Every lane of the issuing warp runs it, so that its arithmetic is uniform; `leader`
+// issues.
+__device__ __forceinline__ void issue3(bool leader, uint32_t d_tmem, bool a_tmem, uint32_t a_hi, uint32_t a_lo, int K,
+                                       uint32_t b_hi, uint32_t b_lo, int N, bool b_mn, uint32_t b_kstride,
+                                       uint32_t b_lbo, uint32_t b_sbo) {
+    const uint32_t idesc = tc::idesc_bf16(N, b_mn ? 1 : 0);
+    uint64_t b0 = tc::smem_desc(b_hi, b_lbo, b_sbo), b1 = tc::smem_desc(b_lo, b_lbo, b_sbo);
+    const uint64_t bstep = b_kstride >> 4;
+    if (a_tmem) {
+#pragma unroll 2
+        for (int ks = 0; ks < K / 16; ++ks) {
+            if (leader) {
+                tc::mma_bf16_ts(d_tmem, a_hi, b0, idesc, ks > 0 ? 1u : 0u);
+                tc::mma_bf16_ts(d_tmem, a_hi, b1, idesc, 1u);
+                tc::mma_bf16_ts(d_tmem, a_lo, b0, idesc, 1u);
+            }
+            a_hi += 8, a_lo += 8, b0 += bstep, b1 += bstep;
+        }
+    } else {
+        uint64_t a0 = tc::smem_desc(a_hi, 128, (uint32_t)K * 16), a1 = tc::smem_desc(a_lo, 128, (uint32_t)K * 16);
+#pragma unroll 2
+        for (int ks = 0; ks < K / 16; ++ks) {
+            if (leader) {
+                tc::mma_bf16(d_tmem, a0, b0, idesc, ks > 0 ? 1u : 0u);
+                tc::mma_bf16(d_tmem, a0, b1, idesc, 1u);
+                tc::mma_bf16(d_tmem, a1, b0, idesc, 1u);
+            }
+            a0 += 16, a1 += 16, b0 += bstep, b1 += bstep;
+        }
+    }
+}
+
+// z[0..8) += b[0..8), two sums an instruction.
+__device__ __forceinline__ void bias8(const float *b, float *z) {
+    const float4 b0 = reinterpret_cast<const float4 *>(b)[0], b1 = reinterpret_cast<const float4 *>(b)[1];
+    const float2 bb[4] = {make_float2(b0.x, b0.y), make_float2(b0.z, b0.w), make_float2(b1.x, b1.y),
+                          make_float2(b1.z, b1.w)};
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const float2 r = add2(make_float2(z[2 * k], z[2 * k + 1]), bb[k]);
+        z[2 * k] = r.x, z[2 * k + 1] = r.y;
+    }
+}
+
+// A thread's chunk at taddr and, with `two`, the one 16 columns on: one wait for both.
+__device__ __forceinline__ void ld_chunks(uint32_t taddr, bool two, float *z) {
+    uint32_t r[16];
+    tc::tmem_ld8_issue(taddr, r);
+    if (two) tc::tmem_ld8_issue(taddr + 16, r + 8);
+    tc::tmem_wait_ld<16>(r, z);
+}
+__device__ __forceinline__ void ld_chunks2(uint32_t ta, uint32_t tb, bool two, float *za, float *zb) {
+    uint32_t r[32];
+    tc::tmem_ld8_issue(ta, r);
+    tc::tmem_ld8_issue(tb, r + 16);
+    if (two) tc::tmem_ld8_issue(ta + 16, r + 8), tc::tmem_ld8_issue(tb + 16, r + 24);
+    float z[32];
+    tc::tmem_wait_ld<32>(r, z);
+#pragma unroll
+    for (int k = 0; k < 16; ++k) za[k] = z[k], zb[k] = z[16 + k];
+}
+
+template <int ACT, bool TMEM_A>
+__global__ void __launch_bounds__(kPThreads, 1) k_mlp_pair(const float *g_rows, const long long *d_np, long long cap,
+                                                          AdjNet net, const float *w, const char *wsplit,
+                                                          float *y_rows, float *dg_rows) {
+    extern __shared__ __align__(128) char smem_raw[];
+    __shared__ uint64_t mbar[2], ready_s[2], wfull_s, wfree_s, done_s;
+    __shared__ uint32_t tmem_slot;
+    const int tid = threadIdx.x, warp = tid >> 5, team = tid / kPTeam, tt = tid & (kPTeam - 1);
+    const int p = tt & (kAP - 1), h = tt / kAP;
+    char *wbuf = smem_raw + net.pair_wbuf;
+    float *par = reinterpret_cast<float *>(smem_raw + net.pair_par);
+    float *eps = reinterpret_cast<float *>(smem_raw + net.pair_eps) + (team & 1) * 2 * kAP;
+    char *tile = smem_raw + (TMEM_A ? 0 : (team & 1) * net.pair_tile);
+    const bool a_tmem = TMEM_A && team == 0;
+    for (int L2 = 0; L2 < net.nh; ++L2) {
+        const int N = net.dims[L2 + 1], Np = net.nout[L2];
+        const float *b = w + net.woff[L2] + (size_t)N * net.dims[L2];
+        for (int n = tid; n < Np; n += kPThreads) par[net.bias_off[L2] + n] = n < N ? b[n] : 0.f;
+    }
+    {
+        const int K = net.dims[net.nh];
+        const float *Wl = w + net.woff[net.nh];
+        for (int k = tid; k < kWideMax; k += kPThreads) par[net.bias_off[net.nh] + k] = k < K ? Wl[k] : 0.f;
+        if (tid == 0) par[net.bias_off[net.nh] + kWideMax] = Wl[K];
+    }
+    if (warp == 0) tc::tmem_alloc(&tmem_slot, 512);
+    if (tid == 0) {
+        tc::mbar_init(&mbar[0], 1);
+        tc::mbar_init(&mbar[1], 1);
+        tc::mbar_init(&ready_s[0], 1);
+        tc::mbar_init(&ready_s[1], 1);
+        tc::mbar_init(&wfull_s, 1);
+        tc::mbar_init(&wfree_s, 1);
+        tc::mbar_init(&done_s, 1);
+    }
+    tc::fence_before();
+    __syncthreads();
+    tc::fence_after();
+    const uint32_t wfull = tc::smem_u32(&wfull_s), wfree = tc::smem_u32(&wfree_s);
+    const int nh = net.nh, np = 2 * nh;  // products of a tile: layers 0 .. nh - 1 forward, nh - 1 .. 0 backward
+    auto layer_of = [&](int s) { return s < nh ? s : np - 1 - s; };
+    // the weights change before product s (the same layer's serve the last forward and
+    // the first backward one, and layer 0's the next round's first)
+    auto loads_before = [&](int s, bool first_round) { return s == 0 ? first_round : s != nh; };
+    const long long P = min(*d_np, cap);
+    const long long ntiles = (P + kAP - 1) / kAP;
+    const long long step = 2LL * gridDim.x;
+    const long long rounds = blockIdx.x < ntiles ? (ntiles - blockIdx.x + step - 1) / step : 0;
+    bool gave_up = false, aborted = false;
+    const uint32_t a_hi = tmem_slot + (uint32_t)(2 * net.pair_d), a_lo = a_hi + (uint32_t)(net.pair_d / 2);  // TMEM_A
+    if (warp == 2 * kPTeam / 32) {  // weights
+        if (tid == 2 * kPTeam) {
+            uint32_t fphase = 0, loads = 0;
+            for (long long r = 0; r < rounds && !gave_up; ++r)
+                for (int s = 0; s < np && !gave_up; ++s) {
+                    if (!loads_before(s, r == 0)) continue;
+                    if (loads > 0) {
+                        if (!tc::mbar_wait(wfree, fphase)) gave_up = true;
+                        fphase ^= 1u;
+                    }
+                    if (gave_up) break;
+                    const int L2 = layer_of(s);
+                    const uint32_t bytes = (uint32_t)(4 * net.nout[L2] * net.kin[L2]);
+                    tc::mbar_arrive_expect_tx(wfull, bytes);
+                    tc::bulk_g2s(tc::smem_u32(wbuf), wsplit + net.wsm_off[L2], bytes, wfull);
+                    ++loads;
+                }
+            // no copy may still write shared memory when the block ends
+            if (loads > 0 && !tc::mbar_wait(wfull, (loads - 1) & 1u)) gave_up = true;
+            if (gave_up) atomicOr(&g_amlp_device_error, kErrMbarTimeout);
+        }
+        __syncwarp();
+    } else if (team == 2) {  // products
+        const bool leader = tc::elect_one();
+        const uint32_t wb = tc::smem_u32(wbuf), t0 = tc::smem_u32(smem_raw);
+        const uint32_t tm0 = __shfl_sync(~0u, tmem_slot, 0);
+        uint32_t wphase = 0, rphase = 0;  // both teams' tiles change phase together
+        for (long long r = 0; r < rounds && !gave_up; ++r)
+            for (int s = 0; s < np && !gave_up; ++s) {
+                const int L2 = layer_of(s), Kp = net.kin[L2], Np = net.nout[L2];
+                const bool fwd = s < nh;
+                if (loads_before(s, r == 0)) {
+                    if (!tc::mbar_wait(wfull, wphase)) gave_up = true;
+                    wphase ^= 1u;
+                }
+                // forward: B = W_k (N' = Np, K' = Kp); backward: W_k read as MN-major (N' = Kp, K' = Np)
+                const int N = fwd ? Np : Kp, K = fwd ? Kp : Np;
+                const uint32_t b_lo = wb + (uint32_t)(Np * Kp * 2), ks = fwd ? 256 : 2 * Kp * 16;
+                const uint32_t lbo = fwd ? 128u : (uint32_t)Kp * 16, sbo = fwd ? (uint32_t)Kp * 16 : 128u;
+#pragma unroll
+                for (int tm = 0; tm < 2; ++tm) {
+                    if (blockIdx.x + (2 * r + tm) * gridDim.x >= ntiles) continue;
+                    if (!tc::mbar_wait(tc::smem_u32(&ready_s[tm]), rphase)) gave_up = true;
+                    gave_up = __any_sync(~0u, gave_up);
+                    if (gave_up) break;
+                    tc::fence_after();
+                    const uint32_t d = tm0 + (uint32_t)(tm * net.pair_d);
+                    if (TMEM_A && tm == 0) {
+                        const uint32_t a0 = tm0 + (uint32_t)(2 * net.pair_d);
+                        issue3(leader, d, true, a0, a0 + (uint32_t)(net.pair_d / 2), K, wb, b_lo, N, !fwd, ks, lbo, sbo);
+                    } else {
+                        const uint32_t a0 = t0 + (TMEM_A ? 0 : tm * net.pair_tile);
+                        issue3(leader, d, false, a0, a0 + (uint32_t)(kAP * K * 2), K, wb, b_lo, N, !fwd, ks, lbo, sbo);
+                    }
+                    if (leader) tc::commit(tc::smem_u32(&mbar[tm]));
+                    __syncwarp();
+                }
+                rphase ^= 1u;
+                if (leader && s + 1 < np && loads_before(s + 1, false)) tc::commit(wfree);
+                __syncwarp();
+            }
+        // products may still be in flight
+        if (leader) tc::commit(tc::smem_u32(&done_s));
+        __syncwarp();
+        if (!tc::mbar_wait(tc::smem_u32(&done_s), 0)) gave_up = true;
+        if (gave_up) atomicOr(&g_amlp_device_error, kErrMbarTimeout);
+    } else {
+        const uint32_t bar = tc::smem_u32(&mbar[team]);
+        const uint32_t dcol = tmem_slot + (uint32_t)(team * net.pair_d);  // this team's product region
+        const uint32_t lane_base = (uint32_t)((warp & 3) * 32) << 16;
+        const uint32_t ready = tc::smem_u32(&ready_s[team]);
+        constexpr bool relu = ACT == AMLP_ACT_RELU;
+        auto dfcol = [&](int k) {  // act'(z_k), smooth activations
+            return tmem_slot + (uint32_t)(2 * net.pair_d + (team * (nh - 1) + k) * net.wmax);
+        };
+        uint32_t phase = 0;
+        const uint32_t row8 = (p & 7) * 16, rows = p >> 3;
+        auto store_a = [&](int K, int c0, const float *v) {
+            uint4 hi, lo;
+            split8(v, hi, lo);
+            if (a_tmem) {
+                tc::tmem_st4(a_hi + lane_base + c0 / 2, hi);
+                tc::tmem_st4(a_lo + lane_base + c0 / 2, lo);
+            } else {
+                char *dst = tile + row8 + rows * (K * 16) + c0 * 16;  // tc::kmajor_offset(p, c0, K)
+                *reinterpret_cast<uint4 *>(dst) = hi;
+                *reinterpret_cast<uint4 *>(dst + kAP * K * 2) = lo;
+            }
+        };
+        // the end of a stage that wrote the operand tile or read TMEM
+        auto stage_end = [&]() {
+            if (a_tmem || !relu) tc::tmem_wait_st();
+            tc::fence_before();
+            tc::fence_async_smem();
+            aborted = pair_sync_or(team, gave_up);
+        };
+        for (long long r = 0; r < rounds && !aborted; ++r) {
+            const long long tl = blockIdx.x + (2 * r + team) * gridDim.x;
+            if (tl >= ntiles) break;  // no tile in the last round
+            const long long r0 = tl * kAP;
+            const int valid = (int)min((long long)kAP, P - r0), Kg = net.kin[0];
+            if (tt == 0 && tl + step < ntiles) {  // the next tile's descriptor rows into L2
+                const long long n0 = (tl + step) * kAP;
+                tc::bulk_prefetch_l2(g_rows + n0 * net.g_ld, (uint32_t)(min((long long)kAP, P - n0) * net.g_ld * 4));
+            }
+            for (int c0 = 8 * h; c0 < Kg; c0 += 16) {
+                float v[8];
+                const float *src = g_rows + (r0 + p) * net.g_ld + c0;
+                const float4 zero4 = make_float4(0.f, 0.f, 0.f, 0.f);
+                const float4 lo4 = p < valid ? reinterpret_cast<const float4 *>(src)[0] : zero4;
+                const float4 hi4 = p < valid ? reinterpret_cast<const float4 *>(src)[1] : zero4;
+                v[0] = lo4.x, v[1] = lo4.y, v[2] = lo4.z, v[3] = lo4.w;
+                v[4] = hi4.x, v[5] = hi4.y, v[6] = hi4.z, v[7] = hi4.w;
+                store_a(Kg, c0, v);
+            }
+            stage_end();
+            uint32_t m[9];  // ReLU: act'(z) bits of hidden layers 0, 1, 2 (this thread's chunks)
+            for (int s = 0; s < np; ++s) {
+                const int L2 = layer_of(s), Kp = net.kin[L2], Np = net.nout[L2];
+                const bool fwd = s < nh;
+                if (!aborted) {
+                    if (tt == 0) tc::mbar_arrive(ready);
+                    if (!tc::mbar_wait(bar, phase)) gave_up = true;
+                    phase ^= 1u;
+                    __syncwarp();
+                    tc::fence_after();
+                }
+                // Columns in chunks of 8, c0 = 8 h, 8 h + 16, ...; two of them at a time.
+                const bool last = L2 == nh - 1;
+                if (fwd) {
+                    const float *bias = par + net.bias_off[L2], *wl = par + net.bias_off[nh];
+                    uint32_t w0 = 0, w1 = 0, w2 = 0;
+                    float esum = 0.f;
+                    auto chunk = [&](int c0, float *z, uint32_t &b8) {
+                        float v[8];
+                        bias8(bias + c0, z);
+                        if (last) {
+                            float ww[8];
+                            *reinterpret_cast<float4 *>(ww) = *reinterpret_cast<const float4 *>(wl + c0);
+                            *reinterpret_cast<float4 *>(ww + 4) = *reinterpret_cast<const float4 *>(wl + c0 + 4);
+#pragma unroll
+                            for (int k = 0; k < 8; ++k) {
+                                float fz, dfz;
+                                act_pair<ACT>(z[k], fz, dfz);
+                                esum = fmaf(ww[k], fz, esum);
+                                v[k] = ww[k] * dfz;
+                            }
+                        } else if (relu) {
+#pragma unroll
+                            for (int k = 7; k >= 0; --k) {
+                                v[k] = fmaxf(z[k], 0.f);
+                                b8 = __funnelshift_l(__float_as_uint(0.f - z[k]), b8, 1);  // its sign: z > 0
+                            }
+                        } else {
+                            float dv[8];
+#pragma unroll
+                            for (int k = 0; k < 8; ++k) act_pair<ACT>(z[k], v[k], dv[k]);
+                            tc::tmem_st8(dfcol(L2) + lane_base + c0, dv);  // for the backward
+                        }
+                        store_a(Np, c0, v);  // the MMA that read the tile is complete
+                    };
+                    for (int j = 0, c0 = 8 * h; c0 < Np; j += 2, c0 += 32) {
+                        float z[16];
+                        const bool two = c0 + 16 < Np;
+                        ld_chunks(dcol + lane_base + c0, two, z);
+                        uint32_t b8 = 0;
+                        if (two) chunk(c0 + 16, z + 8, b8);
+                        chunk(c0, z, b8);
+                        if (relu) {  // 16 bits a step: w0 steps 0, 1; w1 steps 2, 3; w2 step 4
+                            b8 <<= 8 * (j & 2);
+                            if (j < 4) w0 |= b8;
+                            else if (j < 8) w1 |= b8;
+                            else w2 |= b8;
+                        }
+                    }
+                    if (last) eps[h * kAP + p] = esum;
+                    else if (relu) {
+                        if (L2 == 0) m[0] = w0, m[1] = w1, m[2] = w2;
+                        else if (L2 == 1) m[3] = w0, m[4] = w1, m[5] = w2;
+                        else m[6] = w0, m[7] = w1, m[8] = w2;
+                    }
+                } else if (L2 > 0) {
+                    uint32_t w0 = 0, w1 = 0, w2 = 0;
+                    if (relu) {
+                        if (L2 == 1) w0 = m[0], w1 = m[1], w2 = m[2];
+                        else if (L2 == 2) w0 = m[3], w1 = m[4], w2 = m[5];
+                        else w0 = m[6], w1 = m[7], w2 = m[8];
+                    }
+                    for (int j = 0, c0 = 8 * h; c0 < Kp; j += 2, c0 += 32) {
+                        const bool two = c0 + 16 < Kp;
+                        float z[16];
+                        if (relu) {
+                            ld_chunks(dcol + lane_base + c0, two, z);
+                            const uint32_t b8 = (j < 4 ? w0 : (j < 8 ? w1 : w2)) >> (8 * (j & 2));
+#pragma unroll
+                            for (int k = 0; k < 16; ++k) z[k] = (b8 >> k) & 1u ? z[k] : 0.f;
+                        } else {
+                            float df[16];
+                            ld_chunks2(dcol + lane_base + c0, dfcol(L2 - 1) + lane_base + c0, two, z, df);
+#pragma unroll
+                            for (int k = 0; k < 16; ++k) z[k] *= df[k];
+                        }
+                        store_a(Kp, c0, z);
+                        if (two) store_a(Kp, c0 + 16, z + 8);
+                    }
+                } else {
+                    float4 *dst = reinterpret_cast<float4 *>(dg_rows + (r0 + p) * net.gp);
+                    for (int c0 = 8 * h; c0 < Kp; c0 += 32) {
+                        const bool two = c0 + 16 < Kp;
+                        float z[16];
+                        ld_chunks(dcol + lane_base + c0, two, z);
+                        if (p < valid) {
+                            dst[c0 / 4] = make_float4(z[0], z[1], z[2], z[3]);
+                            dst[c0 / 4 + 1] = make_float4(z[4], z[5], z[6], z[7]);
+                            if (two) {
+                                dst[c0 / 4 + 4] = make_float4(z[8], z[9], z[10], z[11]);
+                                dst[c0 / 4 + 5] = make_float4(z[12], z[13], z[14], z[15]);
+                            }
+                        }
+                    }
+                }
+                stage_end();
+                if (fwd && last && tt < kAP && p < valid)
+                    y_rows[r0 + p] = par[net.bias_off[nh] + kWideMax] + eps[p] + eps[kAP + p];
+            }
+        }
+        if (tt == 0 && (aborted || gave_up)) atomicOr(&g_amlp_device_error, kErrMbarTimeout);
+        __syncwarp();
+    }
+    tc::fence_before();
+    __syncthreads();
+    if (warp == 0) {
+        tc::fence_after();
+        tc::tmem_dealloc(tmem_slot, 512);
     }
 }
 
@@ -1553,9 +1961,9 @@ extern "C" amlp_status amlp_multi_forces_adjoint(const float *d_pos, const float
 }
 
 
-constexpr size_t kMlpSmemMax = 226 * 1024;  // dynamic shared memory of k_mlp_grad
+constexpr size_t kMlpSmemMax = 226 * 1024;  // dynamic shared memory of k_mlp_grad and k_mlp_pair
 
-// The net of the wide path and k_mlp_grad's geometry: Kg = padded descriptor
+// The net of the wide path and its kernels' geometry: Kg = padded descriptor
 // width (the first layer's K), g_ld = row stride of the g rows.
 static amlp_status wide_net(const amlp_mlp *mlp, int Kg, int g_ld, AdjNet *net) {
     const int nh = mlp->n_layers - 1;
@@ -1602,6 +2010,37 @@ static amlp_status wide_net(const amlp_mlp *mlp, int Kg, int g_ld, AdjNet *net) 
     net->prefetch_g = with_g <= kMlpSmemMax ? 1 : 0;
     net->smem = (int)(net->prefetch_g ? with_g : o);
     if ((size_t)net->smem > kMlpSmemMax) return AMLP_ERR_UNSUPPORTED;
+    // two tiles in flight (k_mlp_pair) where both operand tiles fit beside a layer's weights
+    // (faster at every width measured: 128 x 2 silu 490 -> 364 us, 150 x 4 ReLU with the first
+    // tile in TMEM 960 -> 627 us); the other nets take k_mlp_grad. TMEM regions start at
+    // multiples of 32 columns.
+    const size_t tile = align_up((size_t)2 * kAP * net->zbw * 2, 128);
+    const size_t rest = align_up((size_t)wbytes, 128) + align_up((size_t)par * 4, 128) + (size_t)4 * kAP * 4;
+    const int df = net->relu_bits ? 0 : 2 * (nh - 1) * net->wmax;
+    net->pair_d = (int)align_up((size_t)net->zbw, 32);
+    net->pair = 0;
+    if (2 * tile + rest <= kMlpSmemMax && 2 * net->pair_d + df <= 512) net->pair = 1;
+    else if (net->relu_bits && tile + rest <= kMlpSmemMax && 3 * net->pair_d <= 512) net->pair = 2;
+    net->pair_tile = (int)tile;
+    net->pair_wbuf = (int)(net->pair == 1 ? 2 * tile : tile);
+    net->pair_par = net->pair_wbuf + (int)align_up((size_t)wbytes, 128);
+    net->pair_eps = net->pair_par + (int)align_up((size_t)par * 4, 128);
+    net->pair_smem = net->pair_eps + 4 * kAP * 4;
+    return AMLP_OK;
+}
+
+// The net pass over the g rows: the weights split once, then k_mlp_pair or k_mlp_grad.
+static amlp_status launch_net(const AdjNet &net, const float *g_rows, const long long *d_npairs, long long cap,
+                              const float *d_w, char *wsplit, float *y_rows, float *dg_rows, cudaStream_t s) {
+    k_split_weights<<<kNumSM, 128, 0, s>>>(net, d_w, wsplit);
+    auto kern = k_mlp_grad;
+    if (net.pair == 2) kern = k_mlp_pair<AMLP_ACT_RELU, true>;
+    else if (net.pair && net.relu_bits) kern = k_mlp_pair<AMLP_ACT_RELU, false>;
+    else if (net.pair) kern = net.act == AMLP_ACT_TANH ? k_mlp_pair<AMLP_ACT_TANH, false> : k_mlp_pair<AMLP_ACT_SILU, false>;
+    const int smem = net.pair ? net.pair_smem : net.smem;
+    AMLP_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    kern<<<kNumSM, net.pair ? kPThreads : kMThreads, smem, s>>>(g_rows, d_npairs, cap, net, d_w, wsplit, y_rows,
+                                                               dg_rows);
     return AMLP_OK;
 }
 
@@ -1692,7 +2131,6 @@ static amlp_status launch_adjoint_wide(const float *d_pos, const float *d_quat, 
         float *y_rows = c.take<float>((size_t)cap);
         char *wsplit = c.take<char>(kWeightSplitBytes);
         if (!c.ok()) return AMLP_ERR_WORKSPACE;
-        AMLP_CHECK_CUDA(cudaFuncSetAttribute(k_mlp_grad, cudaFuncAttributeMaxDynamicSharedMemorySize, net.smem));
         const int npts = nep->npts;
         auto fwd = k2 ? direct::k_desc_direct_fwd<11, 11, 10> : direct::k_desc_direct_fwd<11, 9, 4>;
         auto bwd = k2 ? direct::k_desc_direct_bwd<11, 11, 10> : direct::k_desc_direct_bwd<11, 9, 4>;
@@ -1701,8 +2139,7 @@ static amlp_status launch_adjoint_wide(const float *d_pos, const float *d_quat, 
                                 (const float *)nep->d_pts, npts, inv_rc, g_rows, grow)))
             return st;
         stage_mark(1, s);
-        k_split_weights<<<kNumSM, 128, 0, s>>>(net, mlp->d_w, wsplit);
-        k_mlp_grad<<<kNumSM, kMThreads, net.smem, s>>>(g_rows, d_npairs, cap, net, mlp->d_w, wsplit, y_rows, dg_rows);
+        if ((st = launch_net(net, g_rows, d_npairs, cap, mlp->d_w, wsplit, y_rows, dg_rows, s))) return st;
         stage_mark(2, s);
         if ((st = launch_direct(bwd, cap, npts, s, d_pos, d_quat, box, d_pairs, d_npairs, cap,
                                 (const float *)nep->d_pts, npts, inv_rc, nep->en_min, rng, (const float *)dg_rows, gp,
@@ -1720,7 +2157,6 @@ static amlp_status launch_adjoint_wide(const float *d_pos, const float *d_quat, 
     float *a_rows = c.take<float>(adj_a_bytes(cap) / 4);
     const int npts = nep->npts;
     const size_t smem_desc = wide_desc_smem(npts);
-    const size_t smem_mlp = (size_t)net.smem;
     if (npts > kHarmonicMaxPts) return AMLP_ERR_UNSUPPORTED;
     using Cfg = NepCfg<10, 8, 4, 12>;
     const bool multi = d_rep != nullptr;
@@ -1728,14 +2164,12 @@ static amlp_status launch_adjoint_wide(const float *d_pos, const float *d_quat, 
     auto bwd = multi ? k_adj_desc<Cfg, true, true> : k_adj_desc<Cfg, false, true>;
     AMLP_CHECK_CUDA(cudaFuncSetAttribute(fwd, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_desc));
     AMLP_CHECK_CUDA(cudaFuncSetAttribute(bwd, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_desc));
-    AMLP_CHECK_CUDA(cudaFuncSetAttribute(k_mlp_grad, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_mlp));
     stage_mark(0, s);
     fwd<<<2 * kNumSM, kDThreads, smem_desc, s>>>(d_pos, d_quat, box, d_pairs, d_npairs, cap, nep->d_pts, npts, inv_rc,
                                              nep->en_min, rng, g_rows, kGRow, nullptr, nullptr, nullptr, clip, d_F,
                                              d_T, d_pe, d_rep, d_rp, a_rows);
     stage_mark(1, s);
-    k_split_weights<<<kNumSM, 128, 0, s>>>(net, mlp->d_w, wsplit);
-    k_mlp_grad<<<kNumSM, kMThreads, smem_mlp, s>>>(g_rows, d_npairs, cap, net, mlp->d_w, wsplit, y_rows, dg_rows);
+    if ((st = launch_net(net, g_rows, d_npairs, cap, mlp->d_w, wsplit, y_rows, dg_rows, s))) return st;
     stage_mark(2, s);
     bwd<<<2 * kNumSM, kDThreads, smem_desc, s>>>(d_pos, d_quat, box, d_pairs, d_npairs, cap, nep->d_pts, npts, inv_rc,
                                              nep->en_min, rng, nullptr, kGP, dg_rows, y_rows, d_wt, clip, d_F, d_T,

@@ -45,6 +45,17 @@ __device__ __forceinline__ void mma_bf16(uint32_t d_tmem, uint64_t adesc, uint64
         "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate));
 }
 
+// The same with A in TMEM: row m in lane m, elements (2 c, 2 c + 1) of its K in
+// 32-bit column c.
+__device__ __forceinline__ void mma_bf16_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t bdesc, uint32_t idesc,
+                                            uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}\n" ::"r"(d_tmem),
+        "r"(a_tmem), "l"(bdesc), "r"(idesc), "r"(accumulate));
+}
+
 __device__ __forceinline__ void commit(uint32_t mbar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(mbar)
                  : "memory");
@@ -93,6 +104,13 @@ __device__ __forceinline__ void tmem_st8(uint32_t taddr, const float *v) {
                  : "memory");
 }
 
+// 4 consecutive 32-bit columns, the same.
+__device__ __forceinline__ void tmem_st4(uint32_t taddr, const uint4 &v) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x4.b32 [%0], {%1, %2, %3, %4};" ::"r"(taddr), "r"(v.x), "r"(v.y),
+                 "r"(v.z), "r"(v.w)
+                 : "memory");
+}
+
 __device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
 // 8 consecutive 32-bit columns of this thread's TMEM lane.
@@ -137,6 +155,22 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t phase, int limi
     for (int i = 0; i < limit; ++i)
         if (mbar_try_wait(bar, phase)) return true;
     return false;
+}
+
+// True in one lane of the (converged) warp.
+__device__ __forceinline__ bool elect_one() {
+    uint32_t e;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "elect.sync _|p, 0xffffffff;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}\n"
+        : "=r"(e));
+    return e != 0;
+}
+
+// One arrival on the mbarrier.
+__device__ __forceinline__ void mbar_arrive(uint32_t bar) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
 
 // One arrival on the mbarrier that also expects `bytes` of asynchronous copies.
