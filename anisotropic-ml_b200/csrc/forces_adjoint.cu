@@ -555,7 +555,7 @@ __device__ __forceinline__ void split8(const float *v, uint4 &hi, uint4 &lo) {
     for (int k = 0; k < 4; ++k) {
         const __nv_bfloat162 h2 = __floats2bfloat162_rn(v[2 * k], v[2 * k + 1]);
         const float2 hf = __bfloat1622float2(h2);
-        const float2 r = add2(make_float2(v[2 * k], v[2 * k + 1]), make_float2(-hf.x, -hf.y));
+        const float2 r = fma2(hf, make_float2(-1.f, -1.f), make_float2(v[2 * k], v[2 * k + 1]));  // v - hi
         const __nv_bfloat162 l2 = __floats2bfloat162_rn(r.x, r.y);
         h[k] = *reinterpret_cast<const uint32_t *>(&h2);
         l[k] = *reinterpret_cast<const uint32_t *>(&l2);
@@ -1476,27 +1476,30 @@ __global__ void __launch_bounds__(kMThreads, 1) k_mlp_grad(const float *g_rows, 
 
 // The same net pass with two tiles in flight per CTA. k_mlp_grad runs a tile's products
 // and epilogues one after the other: of its 51 k cycles a tile (four 160-wide layers)
-// the tensor cores worked 20 k. Here two teams of eight warps each have a tile of their
+// the tensor cores worked 20 k. Here two teams of twelve warps each have a tile of their
 // own (operand tile, product region, mbarrier), so that one team's epilogue runs under
 // the other's product, and one copy of the running layer's weights serves both.
-//  - Warp 17 issues the products, team 0's then team 1's of each layer, when a team
+//  - The last warp issues the products, team 0's then team 1's of each layer, when a team
 //    signals that its operand tile is written (ready) and the weights are there (wfull).
 //    All its lanes compute the descriptors, so that they stay in uniform registers:
 //    issued by a thread of the team under a divergent branch, between its scheduler's
 //    epilogues, the 30 MMAs of a 160-wide layer took 3.9 k cycles to issue and 2.4 k to run.
-//  - Warp 16 copies the next layer's weights when both products are complete (wfree).
+//  - The warp before it copies the next layer's weights when both products are complete (wfree).
 //  - A team without a tile (last round) is left out of the round.
 // Two 160-wide operand tiles and a layer's weights do not fit shared memory: with TMEM_A
 // the first team's operand tile is in TMEM (bf16 pairs, hi and lo), which ReLU leaves
 // room for (its derivatives are bits in registers). Smooth activations take this kernel
 // when both tiles fit shared memory and both teams' act'(z) fit TMEM; up to two 128-wide
-// hidden layers do. A product is the same sequence of MMAs as in k_mlp_grad. The
-// epilogues, two chunks of 8 columns a step with the activation known at compile time,
-// take 40 % of the issue slots and bound the kernel with the products' latency.
-// Measured against k_mlp_grad: 5,465 tiles of four 150-wide ReLU layers 960 -> 627 us
-// (tensor pipe busy 336 us), 5,715 tiles of two 128-wide silu layers 490 -> 364 us.
-constexpr int kPTeam = 256;
+// hidden layers do. A product is the same sequence of MMAs as in k_mlp_grad. A team's
+// chain of product and epilogue bounds the kernel (the activation is known at compile
+// time, and three column groups per row shorten it: 3 % faster than two; a fourth would
+// pass 1,024 threads), with the weights' copies, 2.7 k cycles for a 160-wide layer.
+// Measured against k_mlp_grad: 5,465 tiles of four 150-wide ReLU layers 960 -> 581 us
+// (tensor pipe busy 336 us), 5,715 tiles of two 128-wide silu layers 490 -> 335 us.
+constexpr int kPG = 3;               // column groups of a team's epilogues
+constexpr int kPTeam = kPG * kAP;
 constexpr int kPThreads = 2 * kPTeam + 64;
+static_assert(kWideMax <= 8 * 8 * kPG, "a thread's chunks of a layer fit two words of bits");
 
 __device__ __forceinline__ bool pair_sync_or(int team, bool v) {
     uint32_t o;
@@ -1557,24 +1560,6 @@ __device__ __forceinline__ void bias8(const float *b, float *z) {
     }
 }
 
-// A thread's chunk at taddr and, with `two`, the one 16 columns on: one wait for both.
-__device__ __forceinline__ void ld_chunks(uint32_t taddr, bool two, float *z) {
-    uint32_t r[16];
-    tc::tmem_ld8_issue(taddr, r);
-    if (two) tc::tmem_ld8_issue(taddr + 16, r + 8);
-    tc::tmem_wait_ld<16>(r, z);
-}
-__device__ __forceinline__ void ld_chunks2(uint32_t ta, uint32_t tb, bool two, float *za, float *zb) {
-    uint32_t r[32];
-    tc::tmem_ld8_issue(ta, r);
-    tc::tmem_ld8_issue(tb, r + 16);
-    if (two) tc::tmem_ld8_issue(ta + 16, r + 8), tc::tmem_ld8_issue(tb + 16, r + 24);
-    float z[32];
-    tc::tmem_wait_ld<32>(r, z);
-#pragma unroll
-    for (int k = 0; k < 16; ++k) za[k] = z[k], zb[k] = z[16 + k];
-}
-
 template <int ACT, bool TMEM_A>
 __global__ void __launch_bounds__(kPThreads, 1) k_mlp_pair(const float *g_rows, const long long *d_np, long long cap,
                                                           AdjNet net, const float *w, const char *wsplit,
@@ -1582,11 +1567,11 @@ __global__ void __launch_bounds__(kPThreads, 1) k_mlp_pair(const float *g_rows, 
     extern __shared__ __align__(128) char smem_raw[];
     __shared__ uint64_t mbar[2], ready_s[2], wfull_s, wfree_s, done_s;
     __shared__ uint32_t tmem_slot;
-    const int tid = threadIdx.x, warp = tid >> 5, team = tid / kPTeam, tt = tid & (kPTeam - 1);
+    const int tid = threadIdx.x, warp = tid >> 5, team = tid / kPTeam, tt = tid - team * kPTeam;
     const int p = tt & (kAP - 1), h = tt / kAP;
     char *wbuf = smem_raw + net.pair_wbuf;
     float *par = reinterpret_cast<float *>(smem_raw + net.pair_par);
-    float *eps = reinterpret_cast<float *>(smem_raw + net.pair_eps) + (team & 1) * 2 * kAP;
+    float *eps = reinterpret_cast<float *>(smem_raw + net.pair_eps) + (team & 1) * kPG * kAP;
     char *tile = smem_raw + (TMEM_A ? 0 : (team & 1) * net.pair_tile);
     const bool a_tmem = TMEM_A && team == 0;
     for (int L2 = 0; L2 < net.nh; ++L2) {
@@ -1730,18 +1715,22 @@ __global__ void __launch_bounds__(kPThreads, 1) k_mlp_pair(const float *g_rows, 
                 const long long n0 = (tl + step) * kAP;
                 tc::bulk_prefetch_l2(g_rows + n0 * net.g_ld, (uint32_t)(min((long long)kAP, P - n0) * net.g_ld * 4));
             }
-            for (int c0 = 8 * h; c0 < Kg; c0 += 16) {
-                float v[8];
-                const float *src = g_rows + (r0 + p) * net.g_ld + c0;
+            const float4 *src = reinterpret_cast<const float4 *>(g_rows + (r0 + p) * net.g_ld);
+            for (int c0 = 8 * h; c0 < Kg; c0 += 16 * kPG) {  // two chunks' loads in flight
                 const float4 zero4 = make_float4(0.f, 0.f, 0.f, 0.f);
-                const float4 lo4 = p < valid ? reinterpret_cast<const float4 *>(src)[0] : zero4;
-                const float4 hi4 = p < valid ? reinterpret_cast<const float4 *>(src)[1] : zero4;
-                v[0] = lo4.x, v[1] = lo4.y, v[2] = lo4.z, v[3] = lo4.w;
-                v[4] = hi4.x, v[5] = hi4.y, v[6] = hi4.z, v[7] = hi4.w;
+                const bool two = c0 + 8 * kPG < Kg;
+                float4 q[4] = {zero4, zero4, zero4, zero4};
+                if (p < valid) {
+                    q[0] = src[c0 / 4], q[1] = src[c0 / 4 + 1];
+                    if (two) q[2] = src[c0 / 4 + 2 * kPG], q[3] = src[c0 / 4 + 2 * kPG + 1];
+                }
+                const float v[16] = {q[0].x, q[0].y, q[0].z, q[0].w, q[1].x, q[1].y, q[1].z, q[1].w,
+                                     q[2].x, q[2].y, q[2].z, q[2].w, q[3].x, q[3].y, q[3].z, q[3].w};
                 store_a(Kg, c0, v);
+                if (two) store_a(Kg, c0 + 8 * kPG, v + 8);
             }
             stage_end();
-            uint32_t m[9];  // ReLU: act'(z) bits of hidden layers 0, 1, 2 (this thread's chunks)
+            uint32_t m[6];  // ReLU: act'(z) bits of hidden layers 0, 1, 2 (this thread's chunks)
             for (int s = 0; s < np; ++s) {
                 const int L2 = layer_of(s), Kp = net.kin[L2], Np = net.nout[L2];
                 const bool fwd = s < nh;
@@ -1752,14 +1741,15 @@ __global__ void __launch_bounds__(kPThreads, 1) k_mlp_pair(const float *g_rows, 
                     __syncwarp();
                     tc::fence_after();
                 }
-                // Columns in chunks of 8, c0 = 8 h, 8 h + 16, ...; two of them at a time.
+                // columns in chunks of 8: c0 = 8 h, 8 h + 8 kPG, ...
                 const bool last = L2 == nh - 1;
                 if (fwd) {
                     const float *bias = par + net.bias_off[L2], *wl = par + net.bias_off[nh];
-                    uint32_t w0 = 0, w1 = 0, w2 = 0;
+                    uint32_t w0 = 0, w1 = 0;
                     float esum = 0.f;
-                    auto chunk = [&](int c0, float *z, uint32_t &b8) {
-                        float v[8];
+                    for (int j = 0, c0 = 8 * h; c0 < Np; ++j, c0 += 8 * kPG) {
+                        float z[8], v[8];
+                        tc::tmem_ld8(dcol + lane_base + c0, z);
                         bias8(bias + c0, z);
                         if (last) {
                             float ww[8];
@@ -1773,11 +1763,15 @@ __global__ void __launch_bounds__(kPThreads, 1) k_mlp_pair(const float *g_rows, 
                                 v[k] = ww[k] * dfz;
                             }
                         } else if (relu) {
+                            uint32_t b8 = 0;
 #pragma unroll
                             for (int k = 7; k >= 0; --k) {
                                 v[k] = fmaxf(z[k], 0.f);
                                 b8 = __funnelshift_l(__float_as_uint(0.f - z[k]), b8, 1);  // its sign: z > 0
                             }
+                            b8 <<= 8 * (j & 3);
+                            if (j < 4) w0 |= b8;
+                            else w1 |= b8;
                         } else {
                             float dv[8];
 #pragma unroll
@@ -1785,70 +1779,55 @@ __global__ void __launch_bounds__(kPThreads, 1) k_mlp_pair(const float *g_rows, 
                             tc::tmem_st8(dfcol(L2) + lane_base + c0, dv);  // for the backward
                         }
                         store_a(Np, c0, v);  // the MMA that read the tile is complete
-                    };
-                    for (int j = 0, c0 = 8 * h; c0 < Np; j += 2, c0 += 32) {
-                        float z[16];
-                        const bool two = c0 + 16 < Np;
-                        ld_chunks(dcol + lane_base + c0, two, z);
-                        uint32_t b8 = 0;
-                        if (two) chunk(c0 + 16, z + 8, b8);
-                        chunk(c0, z, b8);
-                        if (relu) {  // 16 bits a step: w0 steps 0, 1; w1 steps 2, 3; w2 step 4
-                            b8 <<= 8 * (j & 2);
-                            if (j < 4) w0 |= b8;
-                            else if (j < 8) w1 |= b8;
-                            else w2 |= b8;
-                        }
                     }
                     if (last) eps[h * kAP + p] = esum;
                     else if (relu) {
-                        if (L2 == 0) m[0] = w0, m[1] = w1, m[2] = w2;
-                        else if (L2 == 1) m[3] = w0, m[4] = w1, m[5] = w2;
-                        else m[6] = w0, m[7] = w1, m[8] = w2;
+                        if (L2 == 0) m[0] = w0, m[1] = w1;
+                        else if (L2 == 1) m[2] = w0, m[3] = w1;
+                        else m[4] = w0, m[5] = w1;
                     }
                 } else if (L2 > 0) {
-                    uint32_t w0 = 0, w1 = 0, w2 = 0;
+                    uint32_t w0 = 0, w1 = 0;
                     if (relu) {
-                        if (L2 == 1) w0 = m[0], w1 = m[1], w2 = m[2];
-                        else if (L2 == 2) w0 = m[3], w1 = m[4], w2 = m[5];
-                        else w0 = m[6], w1 = m[7], w2 = m[8];
+                        w0 = L2 == 1 ? m[0] : (L2 == 2 ? m[2] : m[4]);
+                        w1 = L2 == 1 ? m[1] : (L2 == 2 ? m[3] : m[5]);
                     }
-                    for (int j = 0, c0 = 8 * h; c0 < Kp; j += 2, c0 += 32) {
-                        const bool two = c0 + 16 < Kp;
-                        float z[16];
+                    for (int j = 0, c0 = 8 * h; c0 < Kp; ++j, c0 += 8 * kPG) {
+                        float z[8];
                         if (relu) {
-                            ld_chunks(dcol + lane_base + c0, two, z);
-                            const uint32_t b8 = (j < 4 ? w0 : (j < 8 ? w1 : w2)) >> (8 * (j & 2));
+                            tc::tmem_ld8(dcol + lane_base + c0, z);
+                            const uint32_t b8 = (j < 4 ? w0 : w1) >> (8 * (j & 3));
 #pragma unroll
-                            for (int k = 0; k < 16; ++k) z[k] = (b8 >> k) & 1u ? z[k] : 0.f;
+                            for (int k = 0; k < 8; ++k) z[k] = (b8 >> k) & 1u ? z[k] : 0.f;
                         } else {
-                            float df[16];
-                            ld_chunks2(dcol + lane_base + c0, dfcol(L2 - 1) + lane_base + c0, two, z, df);
+                            uint32_t r2[16];
+                            float x[16];
+                            tc::tmem_ld8_issue(dcol + lane_base + c0, r2);
+                            tc::tmem_ld8_issue(dfcol(L2 - 1) + lane_base + c0, r2 + 8);
+                            tc::tmem_wait_ld<16>(r2, x);
 #pragma unroll
-                            for (int k = 0; k < 16; ++k) z[k] *= df[k];
+                            for (int k = 0; k < 8; ++k) z[k] = x[k] * x[8 + k];
                         }
                         store_a(Kp, c0, z);
-                        if (two) store_a(Kp, c0 + 16, z + 8);
                     }
                 } else {
                     float4 *dst = reinterpret_cast<float4 *>(dg_rows + (r0 + p) * net.gp);
-                    for (int c0 = 8 * h; c0 < Kp; c0 += 32) {
-                        const bool two = c0 + 16 < Kp;
-                        float z[16];
-                        ld_chunks(dcol + lane_base + c0, two, z);
+                    for (int c0 = 8 * h; c0 < Kp; c0 += 8 * kPG) {
+                        float z[8];
+                        tc::tmem_ld8(dcol + lane_base + c0, z);
                         if (p < valid) {
                             dst[c0 / 4] = make_float4(z[0], z[1], z[2], z[3]);
                             dst[c0 / 4 + 1] = make_float4(z[4], z[5], z[6], z[7]);
-                            if (two) {
-                                dst[c0 / 4 + 4] = make_float4(z[8], z[9], z[10], z[11]);
-                                dst[c0 / 4 + 5] = make_float4(z[12], z[13], z[14], z[15]);
-                            }
                         }
                     }
                 }
                 stage_end();
-                if (fwd && last && tt < kAP && p < valid)
-                    y_rows[r0 + p] = par[net.bias_off[nh] + kWideMax] + eps[p] + eps[kAP + p];
+                if (fwd && last && tt < kAP && p < valid) {
+                    float ysum = par[net.bias_off[nh] + kWideMax];
+#pragma unroll
+                    for (int q = 0; q < kPG; ++q) ysum += eps[q * kAP + p];
+                    y_rows[r0 + p] = ysum;
+                }
             }
         }
         if (tt == 0 && (aborted || gave_up)) atomicOr(&g_amlp_device_error, kErrMbarTimeout);
@@ -2011,11 +1990,11 @@ static amlp_status wide_net(const amlp_mlp *mlp, int Kg, int g_ld, AdjNet *net) 
     net->smem = (int)(net->prefetch_g ? with_g : o);
     if ((size_t)net->smem > kMlpSmemMax) return AMLP_ERR_UNSUPPORTED;
     // two tiles in flight (k_mlp_pair) where both operand tiles fit beside a layer's weights
-    // (faster at every width measured: 128 x 2 silu 490 -> 364 us, 150 x 4 ReLU with the first
-    // tile in TMEM 960 -> 627 us); the other nets take k_mlp_grad. TMEM regions start at
+    // (faster at every width measured: 128 x 2 silu 490 -> 335 us, 150 x 4 ReLU with the first
+    // tile in TMEM 960 -> 581 us); the other nets take k_mlp_grad. TMEM regions start at
     // multiples of 32 columns.
     const size_t tile = align_up((size_t)2 * kAP * net->zbw * 2, 128);
-    const size_t rest = align_up((size_t)wbytes, 128) + align_up((size_t)par * 4, 128) + (size_t)4 * kAP * 4;
+    const size_t rest = align_up((size_t)wbytes, 128) + align_up((size_t)par * 4, 128) + (size_t)2 * kPG * kAP * 4;
     const int df = net->relu_bits ? 0 : 2 * (nh - 1) * net->wmax;
     net->pair_d = (int)align_up((size_t)net->zbw, 32);
     net->pair = 0;
@@ -2025,7 +2004,7 @@ static amlp_status wide_net(const amlp_mlp *mlp, int Kg, int g_ld, AdjNet *net) 
     net->pair_wbuf = (int)(net->pair == 1 ? 2 * tile : tile);
     net->pair_par = net->pair_wbuf + (int)align_up((size_t)wbytes, 128);
     net->pair_eps = net->pair_par + (int)align_up((size_t)par * 4, 128);
-    net->pair_smem = net->pair_eps + 4 * kAP * 4;
+    net->pair_smem = net->pair_eps + 2 * kPG * kAP * 4;
     return AMLP_OK;
 }
 
