@@ -110,6 +110,7 @@ SIGNATURES = {
     "amlp_nlist_build_gated": [_P, _I, _F, _D, _P, _LL, _P, _P, _SZ, _P, _P, _P],
     "amlp_filter_workspace_bytes": [_LL, _PSZ],
     "amlp_pair_filter": [_P, _F, _D, _P, _P, _LL, _P, _P, _P, _SZ, _P],
+    "amlp_pair_filter_zero": [_P, _F, _D, _P, _P, _LL, _P, _P, _P, _SZ, _P, _P, _I, _P, _P],
     "amlp_descriptors": [_P, _P, _F, _P, _LL, ctypes.POINTER(Nep), _P, _P],
     "amlp_mlp_energy": [_P, _LL, ctypes.POINTER(Mlp), _P, _P],
     "amlp_mlp_loss_grad": [_P, _P, _LL, ctypes.POINTER(Mlp), _P, _P, _P],
@@ -136,6 +137,9 @@ SIGNATURES = {
     "amlp_nvt_init": [_P, _P, _P, _P, _I, ctypes.POINTER(Nvt), _I, _P, _P, _SZ, _P],
     "amlp_nvt_step_two": [_P, _P, _P, _P, _P, _P, _P, _P, _I, ctypes.POINTER(Nvt), _P, _P],
     "amlp_nvt_step_one": [_P, _P, _P, _P, _P, _P, _P, _I, ctypes.POINTER(Nvt), _P, _P, _SZ, _P],
+    "amlp_nvt_step": [_P, _P, _P, _P, _P, _P, _P, _P, _P, _I, ctypes.POINTER(Nvt), _P, _P, _SZ, _P],
+    "amlp_multi_pair_filter_zero": [_P, _P, _P, _D, _P, _P, _LL, _P, _P, _P, _SZ, _P, _P, _I, _P, _I, _P],
+    "amlp_multi_nvt_step": [_P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _I, _I, _P, ctypes.POINTER(Nvt), _P, _P],
     "amlp_multi_pair_filter": [_P, _P, _P, _D, _P, _P, _LL, _P, _P, _P, _SZ, _P],
     "amlp_multi_forces_adjoint": [_P, _P, _P, _P, _P, _P, _LL, ctypes.POINTER(Nep), ctypes.POINTER(Mlp),
                                   _P, _P, _P, _P],

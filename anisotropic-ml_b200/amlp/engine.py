@@ -179,7 +179,7 @@ class System:
         else:
             th.xi, th.eta, th.xi_rot, th.eta_rot, th.thermo_fac = THERMOSTAT_SEED
         self.th = torch.frombuffer(bytearray(bytes(th)), dtype=torch.uint8).to(self.device)
-        self.nvt_ws = torch.empty(size_query("amlp_nvt_workspace_bytes", self.N), dtype=torch.uint8,
+        self.nvt_ws = torch.zeros(size_query("amlp_nvt_workspace_bytes", self.N), dtype=torch.uint8,
                                   device=self.device)
         self.nl_ws = torch.empty(size_query("amlp_nlist_workspace_bytes", self.N, self.L, self.r_verlet),
                                  dtype=torch.uint8, device=self.device)
@@ -247,11 +247,10 @@ class System:
         return self.th.data_ptr() + Thermostat.pe.offset
 
     def compute_forces(self, method: str = "fd") -> None:
-        """Zero F, T and the pair-energy sum, filter the pairs, run the force pass."""
-        self.F.zero_()
-        self.T.zero_()
-        self.th[Thermostat.pe.offset:Thermostat.pe.offset + 8].zero_()
-        self.filter_pairs()
+        """Filter the pairs and zero F, T and the pair-energy sum, then run the force pass."""
+        call("amlp_pair_filter_zero", self.pos.data_ptr(), self.L, float(self.shape.cutoff), self.vpairs.data_ptr(),
+             self.nv.data_ptr(), self.cap, self.fpairs.data_ptr(), self.nf.data_ptr(), self.f_ws.data_ptr(),
+             self.f_ws.numel(), self.F.data_ptr(), self.T.data_ptr(), self.N, self._pe_ptr(), _stream())
         args = (self.pos.data_ptr(), self.quat.data_ptr(), self.L, self.fpairs.data_ptr(), self.nf.data_ptr(),
                 self.cap, ctypes.byref(self.nep), ctypes.byref(self.net.struct), self.F.data_ptr(),
                 self.T.data_ptr(), self._pe_ptr(), _stream())
@@ -313,8 +312,10 @@ class System:
         if self.nlist_policy == "displacement":
             self._gated_rebuild()
         self.compute_forces(method)
-        self.integrate_step_two()
-        self.integrate_step_one()
+        call("amlp_nvt_step", self.pos.data_ptr(), self.vel.data_ptr(), self.accel.data_ptr(), self.quat.data_ptr(),
+             self.angmom.data_ptr(), self.dp.data_ptr(), self.mass.data_ptr(), self.F.data_ptr(), self.T.data_ptr(),
+             self.N, ctypes.byref(self.nvt), self.th.data_ptr(), self.nvt_ws.data_ptr(), self.nvt_ws.numel(),
+             _stream())
 
     def step(self, method: str = "fd") -> None:
         """One time step, host-driven (``Sim.step``)."""

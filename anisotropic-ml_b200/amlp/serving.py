@@ -327,12 +327,10 @@ class _Bucket:
     def step_kernels(self) -> None:
         """One step of every system of the bucket: the same launches whatever the active set."""
         st = _stream()
-        self.F.zero_()
-        self.T.zero_()
-        self.pe.zero_()
-        call("amlp_multi_pair_filter", self.pos.data_ptr(), self.rep.data_ptr(), self.rp.data_ptr(),
+        call("amlp_multi_pair_filter_zero", self.pos.data_ptr(), self.rep.data_ptr(), self.rp.data_ptr(),
              float(self.shape.cutoff), self.vpairs.data_ptr(), self.nv.data_ptr(), self.cap, self.fpairs.data_ptr(),
-             self.nf.data_ptr(), self.f_ws.data_ptr(), self.f_ws.numel(), st)
+             self.nf.data_ptr(), self.f_ws.data_ptr(), self.f_ws.numel(), self.F.data_ptr(), self.T.data_ptr(),
+             self.F.shape[0], self.pe.data_ptr(), self.pe.numel(), st)
         args = [self.pos.data_ptr(), self.quat.data_ptr(), self.rep.data_ptr(), self.rp.data_ptr(),
                 self.fpairs.data_ptr(), self.nf.data_ptr(), self.cap, ctypes.byref(self.nep),
                 ctypes.byref(self.net.struct), self.F.data_ptr(), self.T.data_ptr(), self.pe.data_ptr()]
@@ -340,13 +338,10 @@ class _Bucket:
             call("amlp_multi_forces_adjoint", *args, st)
         else:
             call("amlp_multi_forces_adjoint_wide", *args, self.adj_ws.data_ptr(), self.adj_ws.numel(), st)
-        call("amlp_multi_nvt_step_two", self.vel.data_ptr(), self.accel.data_ptr(), self.F.data_ptr(),
-             self.mass.data_ptr(), self.quat.data_ptr(), self.T.data_ptr(), self.angmom.data_ptr(),
-             self.dp.data_ptr(), self.rep.data_ptr(), self.body_cap, self.sys_cap, self.rp.data_ptr(),
-             ctypes.byref(self.prm), self.th.data_ptr(), st)
-        call("amlp_multi_nvt_step_one", self.pos.data_ptr(), self.vel.data_ptr(), self.accel.data_ptr(),
+        call("amlp_multi_nvt_step", self.pos.data_ptr(), self.vel.data_ptr(), self.accel.data_ptr(),
              self.quat.data_ptr(), self.angmom.data_ptr(), self.dp.data_ptr(), self.mass.data_ptr(),
-             self.rep.data_ptr(), self.body_cap, self.rp.data_ptr(), ctypes.byref(self.prm), self.th.data_ptr(), st)
+             self.F.data_ptr(), self.T.data_ptr(), self.rep.data_ptr(), self.body_cap, self.sys_cap,
+             self.rp.data_ptr(), ctypes.byref(self.prm), self.th.data_ptr(), st)
 
 
 @dataclass

@@ -192,12 +192,10 @@ struct amlp_sim {
 
     amlp_status enqueue_forces(int mode, cudaStream_t st) {
         amlp_status s;
-        if ((s = cuda(cudaMemsetAsync(F.p, 0, (size_t)n * 3 * sizeof(float), st), "zero F"))) return s;
-        if ((s = cuda(cudaMemsetAsync(T.p, 0, (size_t)n * 3 * sizeof(float), st), "zero T"))) return s;
-        if ((s = cuda(cudaMemsetAsync(pe(), 0, sizeof(double), st), "zero pe"))) return s;
-        s = amlp_pair_filter(pos.as<float>(), nvt.box, nep.cutoff, vpairs.as<int>(), nv.as<long long>(), cap,
-                             fpairs.as<int>(), nf.as<long long>(), f_ws.p, f_ws.bytes, st);
-        if (s) return lib(s, "amlp_pair_filter");
+        s = amlp_pair_filter_zero(pos.as<float>(), nvt.box, nep.cutoff, vpairs.as<int>(), nv.as<long long>(), cap,
+                                  fpairs.as<int>(), nf.as<long long>(), f_ws.p, f_ws.bytes, F.as<float>(),
+                                  T.as<float>(), n, pe(), st);
+        if (s) return lib(s, "amlp_pair_filter_zero");
         if (mode == AMLP_FORCES_FD) {
             s = amlp_forces_fd(pos.as<float>(), quat.as<float>(), nvt.box, fpairs.as<int>(), nf.as<long long>(), cap,
                                &nep, &mlp, F.as<float>(), T.as<float>(), pe(), st);
@@ -217,13 +215,10 @@ struct amlp_sim {
     amlp_status enqueue_step(int mode, cudaStream_t st) {
         amlp_status s = enqueue_forces(mode, st);
         if (s) return s;
-        s = amlp_nvt_step_two(vel.as<float>(), accel.as<float>(), F.as<float>(), mass.as<float>(), quat.as<float>(),
-                              T.as<float>(), angmom.as<float>(), dp.as<float>(), n, &nvt, th.as<amlp_thermostat>(), st);
-        if (s) return lib(s, "amlp_nvt_step_two");
-        s = amlp_nvt_step_one(pos.as<float>(), vel.as<float>(), accel.as<float>(), quat.as<float>(),
-                              angmom.as<float>(), dp.as<float>(), mass.as<float>(), n, &nvt, th.as<amlp_thermostat>(),
-                              nvt_ws.p, nvt_ws.bytes, st);
-        return lib(s, "amlp_nvt_step_one");
+        s = amlp_nvt_step(pos.as<float>(), vel.as<float>(), accel.as<float>(), quat.as<float>(), angmom.as<float>(),
+                          dp.as<float>(), mass.as<float>(), F.as<float>(), T.as<float>(), n, &nvt,
+                          th.as<amlp_thermostat>(), nvt_ws.p, nvt_ws.bytes, st);
+        return lib(s, "amlp_nvt_step");
     }
 
     // The state a step changes, saved and restored around the eager warm-up step.
@@ -306,6 +301,7 @@ extern "C" amlp_status amlp_create(const amlp_sim_config *cfg, amlp_sim **out) {
     if (!s) s = h->cuda(cudaStreamCreateWithFlags(&h->cs, cudaStreamNonBlocking), "capture stream");
     if (!s) s = h->cuda(cudaMemset(h->accel.p, 0, n * 3 * sizeof(float)), "state");
     if (!s) s = h->cuda(cudaMemset(h->dp.p, 0, n * 4 * sizeof(float)), "state");
+    if (!s) s = h->cuda(cudaMemset(h->nvt_ws.p, 0, nvt_bytes), "integrator workspace");
     if (s) {
         amlp_destroy(h);
         return s;
@@ -742,14 +738,11 @@ struct amlp_pool {
     amlp_status enqueue_step(cudaStream_t st) {
         const int nrep = (int)sys.size();
         amlp_status s;
-        if ((s = cuda(cudaMemsetAsync(F.p, 0, (size_t)N * 12, st), "zero F")) ||
-            (s = cuda(cudaMemsetAsync(T.p, 0, (size_t)N * 12, st), "zero T")) ||
-            (s = cuda(cudaMemsetAsync(pe.p, 0, (size_t)nrep * 8, st), "zero pe")))
-            return s;
-        s = amlp_multi_pair_filter(pos.as<float>(), rep.as<int>(), rp.as<amlp_replica>(), nep.cutoff, vpairs.as<int>(),
-                                   nv.as<long long>(), cap, fpairs.as<int>(), nf.as<long long>(), f_ws.p, f_ws.bytes,
-                                   st);
-        if (s) return lib(s, "amlp_multi_pair_filter");
+        s = amlp_multi_pair_filter_zero(pos.as<float>(), rep.as<int>(), rp.as<amlp_replica>(), nep.cutoff,
+                                        vpairs.as<int>(), nv.as<long long>(), cap, fpairs.as<int>(),
+                                        nf.as<long long>(), f_ws.p, f_ws.bytes, F.as<float>(), T.as<float>(), N,
+                                        pe.as<double>(), nrep, st);
+        if (s) return lib(s, "amlp_multi_pair_filter_zero");
         if (wide())
             s = amlp_multi_forces_adjoint_wide(pos.as<float>(), quat.as<float>(), rep.as<int>(), rp.as<amlp_replica>(),
                                                fpairs.as<int>(), nf.as<long long>(), cap, &nep, &mlp, F.as<float>(),
@@ -759,14 +752,10 @@ struct amlp_pool {
                                           fpairs.as<int>(), nf.as<long long>(), cap, &nep, &mlp, F.as<float>(),
                                           T.as<float>(), pe.as<double>(), st);
         if (s) return lib(s, "amlp_multi_forces_adjoint");
-        s = amlp_multi_nvt_step_two(vel.as<float>(), accel.as<float>(), F.as<float>(), mass.as<float>(),
-                                    quat.as<float>(), T.as<float>(), angmom.as<float>(), dp.as<float>(), rep.as<int>(),
-                                    N, nrep, rp.as<amlp_replica>(), &prm, th.as<amlp_thermostat>(), st);
-        if (s) return lib(s, "amlp_multi_nvt_step_two");
-        s = amlp_multi_nvt_step_one(pos.as<float>(), vel.as<float>(), accel.as<float>(), quat.as<float>(),
-                                    angmom.as<float>(), dp.as<float>(), mass.as<float>(), rep.as<int>(), N,
-                                    rp.as<amlp_replica>(), &prm, th.as<amlp_thermostat>(), st);
-        return lib(s, "amlp_multi_nvt_step_one");
+        s = amlp_multi_nvt_step(pos.as<float>(), vel.as<float>(), accel.as<float>(), quat.as<float>(),
+                                angmom.as<float>(), dp.as<float>(), mass.as<float>(), F.as<float>(), T.as<float>(),
+                                rep.as<int>(), N, nrep, rp.as<amlp_replica>(), &prm, th.as<amlp_thermostat>(), st);
+        return lib(s, "amlp_multi_nvt_step");
     }
 
     amlp_status save_restore(bool save, cudaStream_t st) {

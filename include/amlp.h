@@ -184,6 +184,12 @@ amlp_status amlp_pair_filter(const float *d_pos, float box, double cutoff,
                              const int *d_vpairs, const long long *d_nverlet, long long cap_verlet,
                              int *d_pairs, long long *d_npairs,
                              void *d_ws, size_t ws_bytes, void *stream);
+/* The same, and the sums of the force pass that follows set to zero in the same
+ * launch: d_F and d_T (N,3), d_pe (1). */
+amlp_status amlp_pair_filter_zero(const float *d_pos, float box, double cutoff,
+                                  const int *d_vpairs, const long long *d_nverlet, long long cap_verlet,
+                                  int *d_pairs, long long *d_npairs, void *d_ws, size_t ws_bytes,
+                                  float *d_F, float *d_T, int n, double *d_pe, void *stream);
 
 /* --------------------------------------------------------------- descriptors
  * g_all of the reference: row v*P + p holds the D descriptors of
@@ -315,6 +321,12 @@ amlp_status amlp_nvt_step_one(float *d_pos, float *d_vel, const float *d_accel,
                               float *d_quat, float *d_angmom, const float *d_dp, const float *d_mass,
                               int n, const amlp_nvt *prm, amlp_thermostat *d_th,
                               void *d_ws, size_t ws_bytes, void *stream);
+/* Step two, then step one, in one launch; the results are theirs. The first four
+ * bytes of d_ws must be zero, as amlp_nvt_init and every step leave them. */
+amlp_status amlp_nvt_step(float *d_pos, float *d_vel, float *d_accel, float *d_quat, float *d_angmom,
+                          float *d_dp, const float *d_mass, const float *d_F, const float *d_T, int n,
+                          const amlp_nvt *prm, amlp_thermostat *d_th, void *d_ws, size_t ws_bytes,
+                          void *stream);
 
 /* --------------------------------------------------------------- many systems in one launch
  * Serving path: the bodies of independent systems (different sizes, boxes,
@@ -325,6 +337,11 @@ amlp_status amlp_nvt_step_one(float *d_pos, float *d_vel, const float *d_accel,
 amlp_status amlp_multi_pair_filter(const float *d_pos, const int *d_rep, const amlp_replica *d_rp, double cutoff,
                                    const int *d_vpairs, const long long *d_nverlet, long long cap_verlet,
                                    int *d_pairs, long long *d_npairs, void *d_ws, size_t ws_bytes, void *stream);
+/* The same, with d_F and d_T (n,3) and d_pe (nrep) set to zero. */
+amlp_status amlp_multi_pair_filter_zero(const float *d_pos, const int *d_rep, const amlp_replica *d_rp, double cutoff,
+                                        const int *d_vpairs, const long long *d_nverlet, long long cap_verlet,
+                                        int *d_pairs, long long *d_npairs, void *d_ws, size_t ws_bytes,
+                                        float *d_F, float *d_T, int n, double *d_pe, int nrep, void *stream);
 amlp_status amlp_multi_forces_adjoint(const float *d_pos, const float *d_quat, const int *d_rep,
                                       const amlp_replica *d_rp, const int *d_pairs, const long long *d_npairs,
                                       long long cap, const amlp_nep *nep, const amlp_mlp *mlp,
@@ -346,6 +363,11 @@ amlp_status amlp_multi_nvt_step_one(float *d_pos, float *d_vel, const float *d_a
                                     float *d_angmom, const float *d_dp, const float *d_mass, const int *d_rep, int n,
                                     const amlp_replica *d_rp, const amlp_nvt *prm, amlp_thermostat *d_th,
                                     void *stream);
+/* Thermostat update, then step two and step one in one launch. */
+amlp_status amlp_multi_nvt_step(float *d_pos, float *d_vel, float *d_accel, float *d_quat, float *d_angmom,
+                                float *d_dp, const float *d_mass, const float *d_F, const float *d_T,
+                                const int *d_rep, int n, int nrep, const amlp_replica *d_rp, const amlp_nvt *prm,
+                                amlp_thermostat *d_th, void *stream);
 
 /* --------------------------------------------------------------- simulation handles
  * A handle owns one system's device state and buffers and runs the reference's
