@@ -116,8 +116,8 @@ __device__ __forceinline__ void radial_basis(float d, float inv_rc, float *f) {
     }
 }
 
-// Descriptor of one point cloud. `pt(a)` returns point a (a < Nd) and
-// `pt.point_sum()` the sum of all Nd points. The D values are written to
+// Descriptor of one point cloud of Nd points: `pt.each(f)` calls f on them in order and
+// `pt.point_sum()` is their sum. The D values are written to
 // g[d * gstride] (a column of a transposed tile). Only the harmonic passes in
 // pass_mask run (bit p: harmonics p KC .. p KC + KC - 1); the radial sums are
 // written with pass 0, and the angular entries hold the sums of the passes run
@@ -147,8 +147,7 @@ __device__ __forceinline__ void nep_descriptor(const PointFn &pt, int Nd, float 
             for (int k2 = 0; k2 < KC / 2; ++k2) A[n][k2] = make_float2(0.f, 0.f);
 #pragma unroll
         for (int n = 0; n < Cfg::NR; ++n) R[n] = 0.f;
-        for (int a = 0; a < Nd; ++a) {
-            float3 p = pt(a);
+        pt.each([&](const float3 p) {
             float rx = p.x - cx, ry = p.y - cy, rz = p.z - cz;
             float d2 = fmaf(rx, rx, fmaf(ry, ry, rz * rz));
             float inv_d = rsqrt_ftz(d2);
@@ -166,7 +165,7 @@ __device__ __forceinline__ void nep_descriptor(const PointFn &pt, int Nd, float 
 #pragma unroll
                 for (int k2 = 0; k2 < KC / 2; ++k2)
                     A[n][k2] = fma2(make_float2(f[n], f[n]), make_float2(Y[k0 + 2 * k2], Y[k0 + 2 * k2 + 1]), A[n][k2]);
-        }
+        });
         if (pass == 0) {
 #pragma unroll
             for (int n = 0; n < Cfg::NR; ++n) g[n * gstride] = R[n];
@@ -241,6 +240,33 @@ struct VariantPoints {
         float3 p = make_float3(B[3 * b], B[3 * b + 1], B[3 * b + 2]);
         if (c2) return make_float3(__fsub_rn(p.x, tx), __fsub_rn(p.y, ty), __fsub_rn(p.z, tz));
         return make_float3(__fadd_rn(p.x, tx), __fadd_rn(p.y, ty), __fadd_rn(p.z, tz));
+    }
+    template <class F>
+    __device__ __forceinline__ void each(const F &f) const {
+        for (int a = 0; a < 2 * h; ++a) f((*this)(a));
+    }
+};
+
+// The same points with the rotated first half read from memory: both halves are
+// points plus a shift (zero for a rotated half), one loop without a branch on the
+// variant. The sum and each point are the ones above to the bit.
+struct StagedPoints {
+    VariantPoints vp;
+    const float *A;  // first half: the rotated copy of variants 4..9, the body's points otherwise
+    __device__ __forceinline__ float3 point_sum() const { return vp.point_sum(); }
+    template <class F>
+    __device__ __forceinline__ void each(const F &f) const {
+        const bool c2 = vp.v >= 7;
+        const float *p = A;
+        float sx = vp.v == 1 ? vp.dx : 0.f, sy = vp.v == 2 ? vp.dx : 0.f, sz = vp.v == 3 ? vp.dx : 0.f;
+#pragma unroll 1
+        for (int half = 0; half < 2; ++half) {
+#pragma unroll 2
+            for (int a = 0; a < vp.h; ++a, p += 3)
+                f(make_float3(__fadd_rn(p[0], sx), __fadd_rn(p[1], sy), __fadd_rn(p[2], sz)));
+            p = c2 ? vp.Ri : vp.Rj;
+            sx = c2 ? -vp.tx : vp.tx, sy = c2 ? -vp.ty : vp.ty, sz = c2 ? -vp.tz : vp.tz;
+        }
     }
 };
 

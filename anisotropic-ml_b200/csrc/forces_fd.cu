@@ -40,9 +40,12 @@ __host__ __device__ inline TileGeom tile_geom(int npts) {
 // Rotated body points of the pairs [p0, p0 + kPT) (clamped to the last pair),
 // the minimum-image translations and the pair indices. The pairs'
 // orientations are read once into shared memory first. The caller's barrier
-// must separate this from the previous use of R, t and ij.
+// must separate this from the previous use of R, t and ij. With V, the first halves
+// of variants 4..9 too: variant v of pair p at V + ((v - 4) kPT + p) vs.
+__device__ __forceinline__ int staged_stride(int npts) { return 3 * npts | 1; }  // odd: no bank conflicts over pairs
 __device__ void load_tile(const float *pos, const float *quat, float L, const int *pairs, long long P, long long p0,
-                          const float *pts_s, const TileGeom &g, float *R, float *t, int *ij) {
+                          const float *pts_s, const TileGeom &g, float *R, float *t, int *ij, float *V = nullptr,
+                          float dteta = 0.f) {
     __shared__ float4 qs[2 * kPT];
     const int nthr = blockDim.x;
     for (int p = threadIdx.x; p < kPT; p += nthr) {
@@ -68,15 +71,24 @@ __device__ void load_tile(const float *pos, const float *quat, float L, const in
         dst[3 * a] = r.x;
         dst[3 * a + 1] = r.y;
         dst[3 * a + 2] = r.z;
+        if (V) {
+#pragma unroll
+            for (int ax = 0; ax < 3; ++ax) {
+                const float3 rr = rotate_ref(variant_quat(4 + ax, dteta), r);
+                float *d = V + ((3 * body + ax) * kPT + p) * staged_stride(g.npts) + 3 * a;
+                d[0] = rr.x, d[1] = rr.y, d[2] = rr.z;
+            }
+        }
     }
 }
 
 // Descriptor of row (variant v, pair p = lane) of the staged tile into
 // gT[d*ld + col], the harmonic passes in pass_mask.
-template <class Cfg>
+template <class Cfg, bool STAGED = false>
 __device__ __forceinline__ void tile_descriptor_row(const float *R, const float *t, const TileGeom &g, float dx,
                                                     float dteta, float inv_rc, float *gT, int ld, int col, int v,
-                                                    unsigned pass_mask = (1u << Cfg::NPASS) - 1u) {
+                                                    unsigned pass_mask = (1u << Cfg::NPASS) - 1u,
+                                                    const float *V = nullptr) {
     const int p = threadIdx.x & 31;
     VariantPoints vp;
     vp.Ri = R + p * g.rs;
@@ -88,7 +100,12 @@ __device__ __forceinline__ void tile_descriptor_row(const float *R, const float 
     vp.v = v;
     vp.dx = dx;
     vp.q = variant_quat(v, dteta);
-    nep_descriptor<Cfg>(vp, g.nd, inv_rc, gT + col, ld, pass_mask);
+    if (STAGED) {  // the rotated halves from V
+        const float *A = v < 4 ? vp.Ri : V + ((v - 4) * kPT + p) * staged_stride(g.npts);
+        nep_descriptor<Cfg>(StagedPoints{vp, A}, g.nd, inv_rc, gT + col, ld, pass_mask);
+    } else {
+        nep_descriptor<Cfg>(vp, g.nd, inv_rc, gT + col, ld, pass_mask);
+    }
 }
 
 // The tile's 10 x kPT descriptor rows from gT (column v kPT + p, row stride ld,
@@ -710,7 +727,17 @@ __device__ __forceinline__ void scatter_tile(const float *fd, const int *ij, int
     }
 }
 
+// STAGED: the rotated halves of variants 4..9 are formed once per tile, in the part of bufB
+// that the descriptor stage leaves free, instead of in both passes of every row; the point
+// loop then has no branch on the variant (20,011 cubes of 26 points: 3,578 -> 3,470 us).
+// Larger clouds, whose copies do not fit there, rotate on the fly. Floats of bufB that the
+// second passes of variants 8 and 9 take, and the most points that fit after them:
 template <class Cfg>
+constexpr int kFdSplit = Cfg::D * 2 * kPT;
+template <class Cfg>
+constexpr int kFdStagedPts = ((kFusedMaxWidth * kRows - kFdSplit<Cfg>) / (6 * kPT) - 1) / 3;
+
+template <class Cfg, bool STAGED>
 __global__ void __launch_bounds__(kFusedThreads, 1) k_forces_fd(const float *pos, const float *quat, float L,
                                                                const int *pairs, const long long *d_np, long long cap,
                                                                const float *pts, int npts, float inv_rc, FdConst c,
@@ -756,10 +783,12 @@ __global__ void __launch_bounds__(kFusedThreads, 1) k_forces_fd(const float *pos
     for (long long tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
         const long long p0 = tile * kPT;
         const int valid = (int)min((long long)kPT, P - p0);
-        load_tile(pos, quat, L, pairs, P, p0, pts_s, g, R, t, ij);
+        float *V = STAGED ? bufB + kFdSplit<Cfg> : nullptr;
+        load_tile(pos, quat, L, pairs, P, p0, pts_s, g, R, t, ij, V, c.dteta);
         __syncthreads();
-        tile_descriptor_row<Cfg>(R, t, g, c.dx, c.dteta, inv_rc, warp < 10 ? bufA : bufB, warp < 10 ? kRows : 2 * kPT,
-                                 warp < 10 ? act_col(threadIdx.x) : threadIdx.x - kRows, dv, dmask);
+        tile_descriptor_row<Cfg, STAGED>(R, t, g, c.dx, c.dteta, inv_rc, warp < 10 ? bufA : bufB,
+                                         warp < 10 ? kRows : 2 * kPT,
+                                         warp < 10 ? act_col(threadIdx.x) : threadIdx.x - kRows, dv, dmask, V);
         __syncthreads();
         if (warp == 8 || warp == 9) {  // the second pass's angular sums (rows NR..D-1; zero where it has none)
             const int col = act_col(threadIdx.x), sc = threadIdx.x - 8 * kPT;
@@ -967,9 +996,10 @@ static amlp_status launch_fd(const float *d_pos, const float *d_quat, float box,
     cudaStream_t s = as_stream(stream);
     int grid = kNumSM;
     if (hyper_kind(nep) == 1) {
-        if ((st = set_smem(k_forces_fd<CfgA>, smem))) return st;
-        k_forces_fd<CfgA><<<grid, kFusedThreads, smem, s>>>(d_pos, d_quat, box, d_pairs, d_npairs, cap, nep->d_pts,
-                                                           nep->npts, inv_rc, c, net, mlp->d_w, d_F, d_T, d_pe, d_e);
+        auto kern = nep->npts <= kFdStagedPts<CfgA> ? k_forces_fd<CfgA, true> : k_forces_fd<CfgA, false>;
+        if ((st = set_smem(kern, smem))) return st;
+        kern<<<grid, kFusedThreads, smem, s>>>(d_pos, d_quat, box, d_pairs, d_npairs, cap, nep->d_pts, nep->npts, inv_rc,
+                                               c, net, mlp->d_w, d_F, d_T, d_pe, d_e);
     } else {
         return AMLP_ERR_UNSUPPORTED;
     }
