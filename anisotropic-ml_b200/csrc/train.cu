@@ -13,17 +13,18 @@
 //   forward   z[r][n]  = b[n] + sum_k W[n][k] a[r][k]  (ascending k, one rounding per
 //             multiply-add), thread = 4 rows x NC columns;
 //   gradient  dW[n][k] = sum_r delta[r][n] a[r][k], thread = NJ x NI weights over all
-//             rows, a warp's lanes on consecutive k: one coalesced reduction per
-//             weight and tile into the caller's gradient buffer;
+//             rows, a warp's lanes 4 n x 8 consecutive k: one reduction per weight and
+//             tile into the caller's gradient buffer, 32 bytes of a row at a time;
 //   deltas    delta_prev[r][k] = act' sum_n W[n][k] delta[r][n], thread as forward,
 //             written over the activations they belong to (ReLU's and tanh's
 //             derivatives follow from the activation; SiLU keeps z beside it).
 // The weights are read through L1 (a warp shares each of them), so that the shared
 // memory holds rows alone: the more rows per tile, the fewer reductions. R is
 // chosen so that the tiles fill whole rounds of the SMs, at most 64.
-// Bound by the L1 that serves both the rows and the weights (72 % of its rate, the
-// multiply-add pipe at 35 %). 16,384 rows of the 47-150-150-150-150-1 ReLU net: 347 us,
-// 21 TFLOP/s. Before, 3,254 us: a thread walked one output column over 32 rows with a
+// Bound by the L1 that serves both the rows and the weights; the forward and the deltas
+// take four fifths of the time, the gradient products the rest (without them 261 of 355
+// us). 16,384 rows of the 47-150-150-150-150-1 ReLU net: 327 us, 22 TFLOP/s. Before
+// the tiles, 3,254 us: a thread walked one output column over 32 rows with a
 // shared-memory load per multiply-add, and every 32 rows paid one reduction per weight.
 #include <algorithm>
 
@@ -53,13 +54,16 @@ __host__ __device__ constexpr int train_ld(int rg) { return 4 * (rg | 1); }
 // acc[i][c] (rows 2 i, 2 i + 1) += sum over k = 0 .. K - 1, ascending, of x[k][rows]
 // times the weight of column c: x points at the thread's four rows of feature 0
 // (features ld apart). ROWS: column c's weights are consecutive floats at w + c col
-// (the forward's, one row of W per column; vec2: 8-byte aligned), otherwise the
+// (the forward's, one row of W per column), otherwise the
 // columns are consecutive and k's weights are the floats at w + k step (the
 // deltas', one row of W per k). The next four k's weights load while four k's
-// multiply-adds issue.
-template <int NC, bool ROWS>
+// multiply-adds issue, VEC floats to a load (the rows' alignment; without ROWS, 4 columns):
+// at compile time, as the loads' registers decide the loop's. 128-wide layers, 16-byte
+// loads: 686 -> 608 us for 50,021 rows of 47-128-128-128-1; 150-wide, 8-byte ones as
+// before, but without the choice inside the loop: 347 -> 323 us.
+template <int NC, bool ROWS, int VEC>
 __device__ __forceinline__ void train_product(float2 (&acc)[2][NC], const float *x, int ld, int K, const float *w,
-                                              int col, int step, bool vec2) {
+                                              int col, int step) {
     const float *p[ROWS ? NC : 1];
     p[0] = w;
     if (ROWS) {
@@ -84,7 +88,21 @@ __device__ __forceinline__ void train_product(float2 (&acc)[2][NC], const float 
         }
     };
     auto load4 = [&](float (&wv)[4][NC]) {
-        if (ROWS && vec2) {
+        if constexpr (ROWS && VEC == 4) {
+#pragma unroll
+            for (int c = 0; c < NC; ++c) {
+                const float4 a = __ldg(reinterpret_cast<const float4 *>(p[c]));
+                wv[0][c] = a.x, wv[1][c] = a.y, wv[2][c] = a.z, wv[3][c] = a.w;
+                p[c] += 4;
+            }
+        } else if constexpr (!ROWS && VEC == 4) {
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const float4 a = __ldg(reinterpret_cast<const float4 *>(p[0]));
+                wv[u][0] = a.x, wv[u][1] = a.y, wv[u][2] = a.z, wv[u][3] = a.w;
+                p[0] += step;
+            }
+        } else if constexpr (ROWS && VEC == 2) {
 #pragma unroll
             for (int c = 0; c < NC; ++c) {
                 const float2 a = __ldg(reinterpret_cast<const float2 *>(p[c]));
@@ -124,6 +142,12 @@ __device__ __forceinline__ void train_product(float2 (&acc)[2][NC], const float 
     }
 }
 
+// Floats per load that the rows of W (K each) are aligned to: 4, 2 or 1.
+__device__ __forceinline__ int train_vec(const float *W, int K) {
+    const uintptr_t a = reinterpret_cast<uintptr_t>(W) | (uintptr_t)K * sizeof(float);
+    return (a & 15) == 0 ? 4 : ((a & 7) == 0 ? 2 : 1);
+}
+
 // Consecutive columns per thread of a layer of n, ncg column groups: 1 to 5, or two
 // groups of 4.
 __device__ __forceinline__ int train_columns(int n, int ncg) {
@@ -155,8 +179,11 @@ __device__ __forceinline__ void train_forward(const TrainNet &net, const TrainTi
         const float bv = __ldg(b + f + c);
         acc[0][c] = acc[1][c] = make_float2(bv, bv);
     }
-    const bool vec2 = (K & 1) == 0 && (reinterpret_cast<uintptr_t>(W) & 7) == 0;
-    train_product<NC, true>(acc, t.sm + net.feat[L] * ld + 4 * t.rg, ld, K, W + (size_t)f * K, K, 0, vec2);
+    const float *x = t.sm + net.feat[L] * ld + 4 * t.rg, *Wf = W + (size_t)f * K;
+    const int vec = train_vec(W, K);
+    if (vec == 4) train_product<NC, true, 4>(acc, x, ld, K, Wf, K, 0);
+    else if (vec == 2) train_product<NC, true, 2>(acc, x, ld, K, Wf, K, 0);
+    else train_product<NC, true, 1>(acc, x, ld, K, Wf, K, 0);
 #pragma unroll
     for (int c = 0; c < NC; ++c) {
         const int n = f + c;
@@ -182,8 +209,16 @@ __device__ __forceinline__ void train_deltas(const TrainNet &net, const TrainTil
     float2 acc[2][NC];
 #pragma unroll
     for (int c = 0; c < NC; ++c) acc[0][c] = acc[1][c] = make_float2(0.f, 0.f);
-    train_product<NC, false>(acc, t.sm + net.feat[L + 1] * ld + 4 * t.rg, ld, N, W + train_first(k0, NC, K), 0, K,
-                             false);
+    const float *x = t.sm + net.feat[L + 1] * ld + 4 * t.rg, *Wk = W + train_first(k0, NC, K);
+    if constexpr (NC == 4) {
+        if (train_vec(W, K) == 4 && (k0 & 3) == 0) {
+            train_product<NC, false, 4>(acc, x, ld, N, Wk, 0, K);
+        } else {
+            train_product<NC, false, 1>(acc, x, ld, N, Wk, 0, K);
+        }
+    } else {
+        train_product<NC, false, 1>(acc, x, ld, N, Wk, 0, K);
+    }
 #pragma unroll
     for (int c = 0; c < NC; ++c) out[c] = make_float4(acc[0][c].x, acc[0][c].y, acc[1][c].x, acc[1][c].y);
 }
@@ -209,25 +244,28 @@ __device__ __forceinline__ void train_store_delta(const TrainNet &net, const Tra
     *dst = make_float4(d[0], d[1], d[2], d[3]);
 }
 
-// dL/dW of layer L from its deltas and inputs: warp w takes rows
-// n = w, w + 16, ... of W, NJ at a time, its lanes the columns
-// k = k0 + lane + 32 i.
-template <int NI>
-__device__ __forceinline__ void train_weights(const TrainNet &net, const TrainTile &t, float *grad, int L, int k0) {
-    constexpr int NJ = 5, nw = kTrainThreads / 32;
+// dL/dW of layer L from its deltas and inputs, in tiles of 4 NJ x 8 NI weights per warp:
+// lane (n, k) of 4 x 8 takes rows n + 4 j and columns k + 8 i. A warp's 16-byte reads of
+// four rows of the activations then touch 8 features (one wavefront) and those of the
+// deltas 4; with all lanes along k, the same 40 multiply-adds took 21 wavefronts instead
+// of 9 and the shared memory bounded them (47-128-128-128-1, 50,021 rows: 608 -> 589 us;
+// the reductions, in 32-byte pieces now, cost the 150-wide net 1 %).
+template <int NI, int NJ>
+__device__ __forceinline__ void train_weights(const TrainNet &net, const TrainTile &t, float *grad, int L) {
+    constexpr int nw = kTrainThreads / 32;
     const int K = net.dims[L], N = net.dims[L + 1], ld = net.ld, R = 4 * net.rg;
-    const int warp = t.tid >> 5, lane = t.tid & 31;
+    const int lane = t.tid & 31, nkb = (K + 8 * NI - 1) / (8 * NI), nnb = (N + 4 * NJ - 1) / (4 * NJ);
     float *gW = grad + net.woff[L];
-    const float *a[NI];
-#pragma unroll
-    for (int i = 0; i < NI; ++i) a[i] = t.sm + (net.feat[L] + min(k0 + lane + 32 * i, K - 1)) * ld;
 #pragma unroll 1
-    for (int n0 = warp; n0 < N; n0 += nw * NJ) {
-        const float *d[NJ];
+    for (int tl = t.tid >> 5; tl < nkb * nnb; tl += nw) {
+        const int nb = tl / nkb, k0 = (tl - nb * nkb) * 8 * NI + (lane & 7), n0 = nb * 4 * NJ + (lane >> 3);
+        const float *a[NI], *d[NJ];
         float2 acc[NJ][NI];
 #pragma unroll
+        for (int i = 0; i < NI; ++i) a[i] = t.sm + (net.feat[L] + min(k0 + 8 * i, K - 1)) * ld;
+#pragma unroll
         for (int j = 0; j < NJ; ++j) {
-            d[j] = t.sm + (net.feat[L + 1] + min(n0 + nw * j, N - 1)) * ld;
+            d[j] = t.sm + (net.feat[L + 1] + min(n0 + 4 * j, N - 1)) * ld;
 #pragma unroll
             for (int i = 0; i < NI; ++i) acc[j][i] = make_float2(0.f, 0.f);
         }
@@ -248,15 +286,22 @@ __device__ __forceinline__ void train_weights(const TrainNet &net, const TrainTi
         }
 #pragma unroll
         for (int j = 0; j < NJ; ++j) {
-            const int n = n0 + nw * j;
+            const int n = n0 + 4 * j;
             if (n >= N) break;
 #pragma unroll
             for (int i = 0; i < NI; ++i) {
-                const int k = k0 + lane + 32 * i;
+                const int k = k0 + 8 * i;
                 if (k < K) atomicAdd(gW + (size_t)n * K + k, acc[j][i].x + acc[j][i].y);
             }
         }
     }
+}
+
+// Multiply-adds per lane and row of a layer's tiles: whole rounds of the warps.
+__device__ __forceinline__ int train_tile_cost(int N, int K, int NI, int NJ) {
+    const int tiles = ((K + 8 * NI - 1) / (8 * NI)) * ((N + 4 * NJ - 1) / (4 * NJ));
+    constexpr int nw = kTrainThreads / 32;
+    return (tiles + nw - 1) / nw * NI * NJ;
 }
 
 // dL/db of layer L.
@@ -330,13 +375,15 @@ __global__ void __launch_bounds__(kTrainThreads, 1) k_mlp_loss_grad(const float 
         }
         __syncthreads();
         for (int L = net.n_layers - 1; L >= 0; --L) {
-            const int K = net.dims[L], ni = (K + 31) / 32;
-            if (ni > 5) {
-                for (int i = 0; i < ni; i += 4) train_weights<4>(net, t, grad, L, 32 * i);
-            } else if (ni == 5) train_weights<5>(net, t, grad, L, 0);
-            else if (ni == 4) train_weights<4>(net, t, grad, L, 0);
-            else if (ni == 3) train_weights<3>(net, t, grad, L, 0);
-            else train_weights<2>(net, t, grad, L, 0);
+            const int K = net.dims[L], N = net.dims[L + 1];
+            // the tile with which the layer's tiles cost the warps least
+            const int c55 = train_tile_cost(N, K, 5, 5), c54 = train_tile_cost(N, K, 5, 4);
+            const int c44 = train_tile_cost(N, K, 4, 4), c34 = train_tile_cost(N, K, 3, 4);
+            const int least = min(min(c55, c54), min(c44, c34));
+            if (c55 == least) train_weights<5, 5>(net, t, grad, L);
+            else if (c54 == least) train_weights<5, 4>(net, t, grad, L);
+            else if (c44 == least) train_weights<4, 4>(net, t, grad, L);
+            else train_weights<3, 4>(net, t, grad, L);
             train_bias(net, t, grad, L);
             if (L == 0) break;
             const int nc = train_columns(K, t.ncg), k0 = t.cg * nc;
