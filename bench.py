@@ -85,7 +85,7 @@ LAUNCHES = {"amlp_nlist_build": 11, "amlp_pair_filter": 2, "amlp_forces_fd": 1, 
 # same bytes per pair), so the roofline's traffic is this figure times the launch's pairs.
 DRAM_BYTES_PER_PAIR = {"adjoint": 5.340928e6 / 436636, "fd": 5.318912e6 / 436636}
 # The wide path (nets wider than 64) stores each pair's descriptor row, harmonic sums and dE/dg in
-# HBM between its three launches: the sum over k_adj_desc forward, k_mlp_grad and k_adj_desc backward
+# HBM between its three launches: the sum over k_adj_desc forward, the net kernel and k_adj_desc backward
 # captured at 32,768 cyl24 bodies (381,342 pairs). The per-pair rows do not depend on the shape or the
 # net, so the figure serves every wide workload.
 DRAM_BYTES_PER_PAIR["adjoint_wide"] = (4.141824e6 + 350.520064e6 + 79.480064e6 + 26.586624e6 + 409.184e6

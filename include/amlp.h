@@ -295,7 +295,7 @@ amlp_status amlp_test_first_wait_limit(int polls);
 /* Stage timing (no reference counterpart): with enable = 1, every later
  * amlp_forces_adjoint_wide / amlp_pair_energy_vjp call records CUDA events on
  * its stream around its three stages: descriptor forward, net forward and
- * backward (k_mlp_grad, with the weight split), descriptor backward. Not for
+ * backward (with the weight split), descriptor backward. Not for
  * calls captured into a CUDA graph. amlp_stage_times waits for the last such
  * call's events and writes the three durations in milliseconds. */
 amlp_status amlp_stage_timing(int enable);
