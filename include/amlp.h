@@ -39,6 +39,7 @@
  *   amlp_forces_adjoint   same call with analytic forces/torques (no reference counterpart)
  *   amlp_nvt_step_two     NVT.integrate_step_two  NVT.py:17-64
  *   amlp_nvt_step_one     NVT.integrate_step_one  NVT.py:12-15, :67-129
+ *   amlp_nvt_step         both of them in one launch
  *   amlp_nvt_init         Sim.move_data_to_device kinetic energies  Sim.py:157-158, :171-180
  *   amlp_device_error     (no reference counterpart: error flags of bounded device waits)
  */
