@@ -162,8 +162,22 @@ __device__ __forceinline__ int train_first(int c0, int nc, int n) { return max(0
 struct TrainTile {
     float *sm;
     int tid, rg, cg, ncg;  // row group (4 rows), column group and their number
+    int nr;                // rows of the batch in the tile
     bool on;               // threads past the last whole column group idle in the products
 };
+
+// The thread's four rows v, zero past the tile's last one. Those rows' forward runs on zero
+// inputs, and a net that overflows there would turn their zero deltas into NaN.
+__device__ __forceinline__ float4 train_rows(const TrainTile &t, float4 v) {
+    const int left = t.nr - 4 * t.rg;
+    if (left < 4) {
+        v.w = 0.f;
+        if (left < 3) v.z = 0.f;
+        if (left < 2) v.y = 0.f;
+        if (left < 1) v.x = 0.f;
+    }
+    return v;
+}
 
 // Layer L forward for NC columns per thread from n0.
 template <int NC>
@@ -192,10 +206,11 @@ __device__ __forceinline__ void train_forward(const TrainNet &net, const TrainTi
         float a[4];
 #pragma unroll
         for (int i = 0; i < 4; ++i) a[i] = last ? z[i] : act_f(net.act, z[i]);
-        *reinterpret_cast<float4 *>(t.sm + (net.feat[L + 1] + n) * ld + 4 * t.rg) = make_float4(a[0], a[1], a[2], a[3]);
+        *reinterpret_cast<float4 *>(t.sm + (net.feat[L + 1] + n) * ld + 4 * t.rg) =
+            train_rows(t, make_float4(a[0], a[1], a[2], a[3]));
         if (!last && net.act == AMLP_ACT_SILU)
             *reinterpret_cast<float4 *>(t.sm + (net.zfeat[L + 1] + n) * ld + 4 * t.rg) =
-                make_float4(z[0], z[1], z[2], z[3]);
+                train_rows(t, make_float4(z[0], z[1], z[2], z[3]));
     }
 }
 
@@ -241,7 +256,7 @@ __device__ __forceinline__ void train_store_delta(const TrainNet &net, const Tra
 #pragma unroll
         for (int i = 0; i < 4; ++i) d[i] *= a[i] > 0.0f ? 1.0f : 0.0f;
     }
-    *dst = make_float4(d[0], d[1], d[2], d[3]);
+    *dst = train_rows(t, make_float4(d[0], d[1], d[2], d[3]));
 }
 
 // dL/dW of layer L from its deltas and inputs, in tiles of 4 NJ x 8 NI weights per warp:
@@ -333,7 +348,7 @@ __global__ void __launch_bounds__(kTrainThreads, 1) k_mlp_loss_grad(const float 
     t.on = t.cg < t.ncg;
     const float inv_b = 1.0f / (float)rows;
     for (long long r0 = (long long)blockIdx.x * R; r0 < rows; r0 += (long long)gridDim.x * R) {
-        const int nr = (int)min((long long)R, rows - r0);
+        const int nr = t.nr = (int)min((long long)R, rows - r0);
         const int D = net.dims[0];
         // the tile's descriptor rows, a warp per row (coalesced); rows past the end are zero
         for (int r = t.tid >> 5; r < R; r += kTrainThreads / 32)
