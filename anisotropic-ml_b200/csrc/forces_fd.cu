@@ -479,8 +479,10 @@ __global__ void __launch_bounds__(kTThreads) k_mlp_tiled(const float *g, long lo
                 // cg sums k = cg, cg + 32, ... in ascending order, 8 rows per thread), the
                 // partial sums meet in the activation buffer and add up in group order
                 // after the bias
-                cp_async_wait<0>();
-                __syncthreads();
+                if (K > ks) {
+                    cp_async_wait<0>();
+                    __syncthreads();
+                }
                 const int rg = t & 15, cg = t >> 4;
                 float part[8];
 #pragma unroll
@@ -530,8 +532,12 @@ __global__ void __launch_bounds__(kTThreads) k_mlp_tiled(const float *g, long lo
             cp_async_wait<0>();  // this layer's second part
             __syncthreads();     // and every thread has read its first part and the bias
             stage_weights(m, w, L + 1, 0, kTSplit, WT, Bs);
-            product(ks, K);
-            __syncthreads();  // every thread has read this layer's inputs and weights
+            // the same for all threads; without a second part, this layer has been read by now (the
+            // barrier saved: 184 -> 174 us for 500,000 rows of 47-16-16-1)
+            if (K > ks) {
+                product(ks, K);
+                __syncthreads();  // every thread has read this layer's inputs and weights
+            }
             stage_weights(m, w, L + 1, kTSplit, kTMaxW, WT, Bs);
             auto write = [&](auto act) {
 #pragma unroll
