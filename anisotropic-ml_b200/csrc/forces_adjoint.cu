@@ -27,8 +27,9 @@ namespace amlp {
 
 __device__ unsigned int g_amlp_device_error = 0;
 // Test hook (amlp_test_first_wait_limit): polls allowed to the first MMA-completion
-// wait of every CTA of k_forces_adjoint; -1 keeps the normal limit. 0 makes that
-// wait give up at once, which exercises the abort path without any fault.
+// wait of every CTA of k_forces_adjoint and k_mlp_grad; -1 keeps the normal limit. 0
+// makes that wait give up at once, which exercises the abort path without any fault
+// (in k_mlp_pair 0 makes the teams give up before their first product).
 __device__ int g_amlp_first_wait_limit = -1;
 
 namespace {
@@ -1216,6 +1217,18 @@ __global__ void k_split_weights(AdjNet net, const float *w, char *dst) {
     }
 }
 
+// y and dE/dg of the tiles tl, tl + step, ... to zero: what a wait that gave up leaves
+// behind is not to be trusted, and with dE/dg zero the pairs exert no force.
+__device__ void drop_rows(long long tl, long long step, long long P, int gp, int first, int stride, float *y_rows,
+                          float *dg_rows) {
+    for (; tl * kAP < P; tl += step) {
+        const long long r0 = tl * kAP;
+        const int valid = (int)min((long long)kAP, P - r0);
+        for (int k = first; k < valid; k += stride) y_rows[r0 + k] = 0.f;
+        for (int k = first; k < valid * gp; k += stride) dg_rows[r0 * gp + k] = 0.f;
+    }
+}
+
 // Net forward and backward over rows of g on the tensor cores (bf16x3 splits,
 // fp32 TMEM accumulators), hidden layers up to 160 wide and up to four of them
 // (the reference's TheEnergyNet(150, 3, D): layer_first and three hidden
@@ -1277,9 +1290,11 @@ __global__ void __launch_bounds__(kMThreads, 1) k_mlp_grad(const float *g_rows, 
     // is issued, the tile loop ends and what is in flight is drained at the end.
     bool gave_up = false, aborted = false;
     int commits = 0;
+    int limit = g_amlp_first_wait_limit >= 0 ? g_amlp_first_wait_limit : tc::kWaitLimit;
     auto wait_mma = [&]() {
         if (aborted) return;  // nothing was issued
-        if (!tc::mbar_wait(bar, phase)) gave_up = true;
+        if (!tc::mbar_wait(bar, phase, limit)) gave_up = true;
+        limit = tc::kWaitLimit;
         phase ^= 1u;
         tc::fence_after();
     };
@@ -1468,6 +1483,7 @@ __global__ void __launch_bounds__(kMThreads, 1) k_mlp_grad(const float *g_rows, 
         if (aborted || !drained) atomicOr(&g_amlp_device_error, kErrMbarTimeout);
     }
     __syncthreads();
+    if (aborted) drop_rows(blockIdx.x, gridDim.x, P, net.gp, tid, kMThreads, y_rows, dg_rows);
     if (warp == 0) {
         tc::fence_after();
         tc::tmem_dealloc(tmem, 512);
@@ -1486,6 +1502,8 @@ __global__ void __launch_bounds__(kMThreads, 1) k_mlp_grad(const float *g_rows, 
 //    epilogues, the 30 MMAs of a 160-wide layer took 3.9 k cycles to issue and 2.4 k to run.
 //  - The warp before it copies the next layer's weights when both products are complete (wfree).
 //  - A team without a tile (last round) is left out of the round.
+//  - A role whose wait gives up sets `quit` and leaves; the others follow, the products in
+//    flight are drained, and the block's rows are zeroed (drop_rows).
 // Two 160-wide operand tiles and a layer's weights do not fit shared memory: with TMEM_A
 // the first team's operand tile is in TMEM (bf16 pairs, hi and lo), which ReLU leaves
 // room for (its derivatives are bits in registers). Smooth activations take this kernel
@@ -1512,6 +1530,16 @@ __device__ __forceinline__ bool pair_sync_or(int team, bool v) {
         : "r"((uint32_t)v), "r"(1 + team), "n"(kPTeam)
         : "memory");
     return o != 0;
+}
+
+// Bounded wait that ends early (false) when another role of the block has given up, as
+// that sets `quit`. It is looked at every 64 polls, to keep the polling itself short.
+__device__ __forceinline__ bool pair_wait(uint32_t bar, uint32_t phase, const volatile int *quit) {
+    for (int i = 0; i < tc::kWaitLimit; i += 64) {
+        if (tc::mbar_wait(bar, phase, 64)) return true;
+        if (*quit) return false;
+    }
+    return false;
 }
 
 // mma3's sequence with the descriptors' steps added to their address fields (a shared-memory
@@ -1567,6 +1595,7 @@ __global__ void __launch_bounds__(kPThreads, 1) k_mlp_pair(const float *g_rows, 
     extern __shared__ __align__(128) char smem_raw[];
     __shared__ uint64_t mbar[2], ready_s[2], wfull_s, wfree_s, done_s;
     __shared__ uint32_t tmem_slot;
+    __shared__ int quit;  // a wait of some role has given up
     const int tid = threadIdx.x, warp = tid >> 5, team = tid / kPTeam, tt = tid - team * kPTeam;
     const int p = tt & (kAP - 1), h = tt / kAP;
     char *wbuf = smem_raw + net.pair_wbuf;
@@ -1594,6 +1623,7 @@ __global__ void __launch_bounds__(kPThreads, 1) k_mlp_pair(const float *g_rows, 
         tc::mbar_init(&wfull_s, 1);
         tc::mbar_init(&wfree_s, 1);
         tc::mbar_init(&done_s, 1);
+        quit = 0;
     }
     tc::fence_before();
     __syncthreads();
@@ -1608,7 +1638,7 @@ __global__ void __launch_bounds__(kPThreads, 1) k_mlp_pair(const float *g_rows, 
     const long long ntiles = (P + kAP - 1) / kAP;
     const long long step = 2LL * gridDim.x;
     const long long rounds = blockIdx.x < ntiles ? (ntiles - blockIdx.x + step - 1) / step : 0;
-    bool gave_up = false, aborted = false;
+    bool gave_up = team < 2 && g_amlp_first_wait_limit == 0, aborted = false;
     const uint32_t a_hi = tmem_slot + (uint32_t)(2 * net.pair_d), a_lo = a_hi + (uint32_t)(net.pair_d / 2);  // TMEM_A
     if (warp == 2 * kPTeam / 32) {  // weights
         if (tid == 2 * kPTeam) {
@@ -1617,7 +1647,7 @@ __global__ void __launch_bounds__(kPThreads, 1) k_mlp_pair(const float *g_rows, 
                 for (int s = 0; s < np && !gave_up; ++s) {
                     if (!loads_before(s, r == 0)) continue;
                     if (loads > 0) {
-                        if (!tc::mbar_wait(wfree, fphase)) gave_up = true;
+                        if (!pair_wait(wfree, fphase, &quit)) gave_up = true;
                         fphase ^= 1u;
                     }
                     if (gave_up) break;
@@ -1629,7 +1659,7 @@ __global__ void __launch_bounds__(kPThreads, 1) k_mlp_pair(const float *g_rows, 
                 }
             // no copy may still write shared memory when the block ends
             if (loads > 0 && !tc::mbar_wait(wfull, (loads - 1) & 1u)) gave_up = true;
-            if (gave_up) atomicOr(&g_amlp_device_error, kErrMbarTimeout);
+            if (gave_up) quit = 1;
         }
         __syncwarp();
     } else if (team == 2) {  // products
@@ -1652,7 +1682,7 @@ __global__ void __launch_bounds__(kPThreads, 1) k_mlp_pair(const float *g_rows, 
 #pragma unroll
                 for (int tm = 0; tm < 2; ++tm) {
                     if (blockIdx.x + (2 * r + tm) * gridDim.x >= ntiles) continue;
-                    if (!tc::mbar_wait(tc::smem_u32(&ready_s[tm]), rphase)) gave_up = true;
+                    if (!pair_wait(tc::smem_u32(&ready_s[tm]), rphase, &quit)) gave_up = true;
                     gave_up = __any_sync(~0u, gave_up);
                     if (gave_up) break;
                     tc::fence_after();
@@ -1675,7 +1705,7 @@ __global__ void __launch_bounds__(kPThreads, 1) k_mlp_pair(const float *g_rows, 
         if (leader) tc::commit(tc::smem_u32(&done_s));
         __syncwarp();
         if (!tc::mbar_wait(tc::smem_u32(&done_s), 0)) gave_up = true;
-        if (gave_up) atomicOr(&g_amlp_device_error, kErrMbarTimeout);
+        if (gave_up) quit = 1;
     } else {
         const uint32_t bar = tc::smem_u32(&mbar[team]);
         const uint32_t dcol = tmem_slot + (uint32_t)(team * net.pair_d);  // this team's product region
@@ -1731,16 +1761,14 @@ __global__ void __launch_bounds__(kPThreads, 1) k_mlp_pair(const float *g_rows, 
             }
             stage_end();
             uint32_t m[6];  // ReLU: act'(z) bits of hidden layers 0, 1, 2 (this thread's chunks)
-            for (int s = 0; s < np; ++s) {
+            for (int s = 0; s < np && !aborted; ++s) {
                 const int L2 = layer_of(s), Kp = net.kin[L2], Np = net.nout[L2];
                 const bool fwd = s < nh;
-                if (!aborted) {
-                    if (tt == 0) tc::mbar_arrive(ready);
-                    if (!tc::mbar_wait(bar, phase)) gave_up = true;
-                    phase ^= 1u;
-                    __syncwarp();
-                    tc::fence_after();
-                }
+                if (tt == 0) tc::mbar_arrive(ready);
+                if (!tc::mbar_wait(bar, phase)) gave_up = true;
+                phase ^= 1u;
+                __syncwarp();
+                tc::fence_after();
                 // columns in chunks of 8: c0 = 8 h, 8 h + 8 kPG, ...
                 const bool last = L2 == nh - 1;
                 if (fwd) {
@@ -1830,7 +1858,7 @@ __global__ void __launch_bounds__(kPThreads, 1) k_mlp_pair(const float *g_rows, 
                 }
             }
         }
-        if (tt == 0 && (aborted || gave_up)) atomicOr(&g_amlp_device_error, kErrMbarTimeout);
+        if (tt == 0 && (aborted || gave_up)) quit = 1;
         __syncwarp();
     }
     tc::fence_before();
@@ -1838,6 +1866,10 @@ __global__ void __launch_bounds__(kPThreads, 1) k_mlp_pair(const float *g_rows, 
     if (warp == 0) {
         tc::fence_after();
         tc::tmem_dealloc(tmem_slot, 512);
+    }
+    if (quit) {
+        if (tid == 0) atomicOr(&g_amlp_device_error, kErrMbarTimeout);
+        drop_rows(blockIdx.x, gridDim.x, P, net.gp, tid, kPThreads, y_rows, dg_rows);
     }
 }
 

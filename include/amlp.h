@@ -286,11 +286,12 @@ amlp_status amlp_mlp_backward(const float *d_g, const float *d_dy, long long row
 amlp_status amlp_device_error(unsigned int *flags, int clear);
 
 /* Test hook (no reference counterpart): the number of polls allowed to the
- * first tensor-core completion wait of every CTA of amlp_forces_adjoint's
- * kernel, so that a test can make that wait give up without a fault: with 0 it
- * gives up at once, the kernel raises bit 1 of amlp_device_error, issues no
- * further MMA, drains the one in flight (normal limit) and frees its tensor
- * memory. -1 restores the normal limit. It applies to later launches. */
+ * first tensor-core completion wait of every CTA of the adjoint force kernels, so
+ * that a test can make that wait give up without a fault: with 0 it gives up at
+ * once (in the wide path's two-tile kernel before the first product is issued),
+ * the kernel raises bit 1 of amlp_device_error, issues no further MMA, drains the
+ * one in flight (normal limit), frees its tensor memory, and the pairs it worked
+ * on exert no force. -1 restores the normal limit. It applies to later launches. */
 amlp_status amlp_test_first_wait_limit(int polls);
 
 /* Stage timing (no reference counterpart): with enable = 1, every later
