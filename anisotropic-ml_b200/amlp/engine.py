@@ -248,9 +248,15 @@ class System:
 
     def compute_forces(self, method: str = "fd") -> None:
         """Filter the pairs and zero F, T and the pair-energy sum, then run the force pass."""
+        self._filter_and_zero()
+        self._force_pass(method)
+
+    def _filter_and_zero(self) -> None:
         call("amlp_pair_filter_zero", self.pos.data_ptr(), self.L, float(self.shape.cutoff), self.vpairs.data_ptr(),
              self.nv.data_ptr(), self.cap, self.fpairs.data_ptr(), self.nf.data_ptr(), self.f_ws.data_ptr(),
              self.f_ws.numel(), self.F.data_ptr(), self.T.data_ptr(), self.N, self._pe_ptr(), _stream())
+
+    def _force_pass(self, method: str) -> None:
         args = (self.pos.data_ptr(), self.quat.data_ptr(), self.L, self.fpairs.data_ptr(), self.nf.data_ptr(),
                 self.cap, ctypes.byref(self.nep), ctypes.byref(self.net.struct), self.F.data_ptr(),
                 self.T.data_ptr(), self._pe_ptr(), _stream())
@@ -312,6 +318,9 @@ class System:
         if self.nlist_policy == "displacement":
             self._gated_rebuild()
         self.compute_forces(method)
+        self._nvt_step()
+
+    def _nvt_step(self) -> None:
         call("amlp_nvt_step", self.pos.data_ptr(), self.vel.data_ptr(), self.accel.data_ptr(), self.quat.data_ptr(),
              self.angmom.data_ptr(), self.dp.data_ptr(), self.mass.data_ptr(), self.F.data_ptr(), self.T.data_ptr(),
              self.N, ctypes.byref(self.nvt), self.th.data_ptr(), self.nvt_ws.data_ptr(), self.nvt_ws.numel(),

@@ -74,9 +74,14 @@ WORKLOADS = {
 HYPERS = (10, 8, 4)
 BOX = None  # explicit box edge (workloads at a given number density instead of a packing fraction)
 
-# kernels launched by each libamlp entry point (for the gpu_launches count)
-LAUNCHES = {"amlp_nlist_build": 11, "amlp_pair_filter": 2, "amlp_forces_fd": 1, "amlp_forces_adjoint": 1,
-            "amlp_nvt_step_two": 2, "amlp_nvt_step_one": 1}
+# kernels launched by each libamlp entry point of a step (for the gpu_launches count)
+LAUNCHES = {"amlp_nlist_build": 12, "amlp_pair_filter_zero": 2, "amlp_forces_fd": 1, "amlp_forces_adjoint": 1,
+            "amlp_forces_adjoint_wide": 4, "amlp_descriptors": 1, "amlp_mlp_energy": 1, "amlp_fd_scatter": 1,
+            "amlp_nvt_step": 1}
+# the entry points of a force pass
+FORCE_CALLS = {"fd": ["amlp_forces_fd"], "adjoint": ["amlp_forces_adjoint"],
+               "adjoint_wide": ["amlp_forces_adjoint_wide"],
+               "fd_split": ["amlp_descriptors", "amlp_mlp_energy", "amlp_fd_scatter"]}
 
 
 # DRAM bytes (read + written) per filtered pair of one force launch, from an ncu capture of
@@ -99,6 +104,7 @@ STAGE_DRAM_BYTES_PER_PAIR = {
     ("k_adj_desc (backward)", 47): (409.184e6 + 5.303552e6) / 381342,
     ("k_mlp_grad", 47): 18.56128e6 / 87256,
     ("k_mlp_grad", 121): (46.54e6 + 0.39e6) / 87257,
+    ("k_mlp_pair", 47): 18.6e6 / 87256,
     ("k_desc_direct_fwd", 47): 1.64e6 / 87256,
     ("k_desc_direct_bwd", 47): 19.54e6 / 87256,
     ("k_desc_direct_fwd", 121): (2.888960e6 + 1.725440e6) / 87257,
@@ -111,6 +117,23 @@ def uses_direct_form(nd: int, hypers=(10, 8, 4)) -> bool:
     hypers (10, 10, 10), and (10, 8, 4) clouds of at most 12 points (the
     library's own choice, kDirectMaxNd47)."""
     return tuple(hypers) != (10, 8, 4) or nd <= 12
+
+
+def net_kernel(D: int, widths, act: str) -> str:
+    """The net kernel of the wide path: two tiles in flight (k_mlp_pair) where their operands fit
+    shared memory, or for ReLU the first one tensor memory, else one (the library's own choice,
+    wide_net: 226 KB of shared memory and 512 tensor-memory columns)."""
+    up = lambda x, a: (x + a - 1) // a * a  # noqa: E731
+    kg = 48 if D <= 48 else 128
+    nout = [up(w, 16) for w in widths]
+    wmax, zb = max(nout), max(kg, max(nout))
+    wbytes = max(4 * n * k for n, k in zip(nout, [kg] + nout))
+    tile = up(512 * zb, 128)
+    rest = up(wbytes, 128) + up(4 * (sum(nout) + 164), 128) + 3072
+    cols, relu = up(zb, 32), act == "relu"
+    both = 2 * tile + rest <= 226 * 1024 and 2 * cols + (0 if relu else 2 * (len(nout) - 1) * wmax) <= 512
+    first_in_tmem = relu and tile + rest <= 226 * 1024 and 3 * cols <= 512
+    return "k_mlp_pair" if both or first_in_tmem else "k_mlp_grad"
 
 
 def descriptor_flops(nd: int, hypers=(10, 8, 4), direct: bool = False) -> float:
@@ -357,6 +380,22 @@ def job_throughput(world: int, n_bodies: int, steps: int, job_ms: float) -> floa
 
 
 # ----------------------------------------------------------------------------- GPU arm
+def engine_step(system, method: str, before_forces=None, after_forces=None) -> int:
+    """One step of the engine (the launches of ``System``'s own), with callbacks around its force
+    pass. Returns the number of kernels launched."""
+    system._filter_and_zero()
+    if before_forces:
+        before_forces()
+    system._force_pass(method)
+    if after_forces:
+        after_forces()
+    system._nvt_step()
+    system.timestep += 1
+    wide = method == "adjoint" and system.adj_ws is not None
+    return sum(LAUNCHES[c] for c in ["amlp_pair_filter_zero", "amlp_nvt_step"] +
+               FORCE_CALLS["adjoint_wide" if wide else method])
+
+
 def _measure(system, method: str, steps: int, warmup: int, dist, dev):
     """Device time of `steps` full steps (L2 flushed between steps, outside the
     events) and of the force kernel inside them. Returns a dict."""
@@ -366,10 +405,7 @@ def _measure(system, method: str, steps: int, warmup: int, dist, dev):
     stream = torch.cuda.current_stream()
     flush = torch.empty(256 * 1024 * 1024, dtype=torch.uint8, device=dev)  # > 126 MB L2
     launches = [0]
-    entry = "amlp_forces_" + ("fd" if method == "fd" else "adjoint")
     wide = method == "adjoint" and system.adj_ws is not None  # beyond the fused kernel: the wide adjoint
-    if wide:
-        entry = "amlp_forces_adjoint_wide"
 
     # Verlet rebuilds: every nlist_every steps counted from the first timed step, so that
     # the timed window starts with one (warm-up steps follow the engine's own schedule)
@@ -384,28 +420,7 @@ def _measure(system, method: str, steps: int, warmup: int, dist, dev):
             system.build_nlist(check=False)
             launches[0] += LAUNCHES["amlp_nlist_build"]
             rebuilds[0] += 1
-        system.F.zero_()
-        system.T.zero_()
-        system.th[_lib.Thermostat.pe.offset:_lib.Thermostat.pe.offset + 8].zero_()
-        system.filter_pairs()
-        if ev_force is not None:
-            ev_force[0].record(stream)
-        args = [system.pos.data_ptr(), system.quat.data_ptr(), system.L, system.fpairs.data_ptr(),
-                system.nf.data_ptr(), system.cap, ctypes.byref(system.nep), ctypes.byref(system.net.struct),
-                system.F.data_ptr(), system.T.data_ptr(), system._pe_ptr()]
-        if wide:
-            args += [system.adj_ws.data_ptr(), system.adj_ws.numel()]
-        if method == "fd_split":  # the reference's data flow: g_all and e_all in HBM, one pair-count read
-            system._forces_split()
-        else:
-            _lib.call(entry, *args, stream.cuda_stream)
-        if ev_force is not None:
-            ev_force[1].record(stream)
-        system.integrate_step_two()
-        system.integrate_step_one()
-        system.timestep += 1
-        launches[0] += (LAUNCHES["amlp_pair_filter"] + (4 if wide else 3 if method == "fd_split" else 1) +
-                        LAUNCHES["amlp_nvt_step_two"] + LAUNCHES["amlp_nvt_step_one"])
+        launches[0] += engine_step(system, method, *(e.record for e in ev_force or ()))
 
     for _ in range(warmup):
         one_step()
@@ -545,8 +560,9 @@ def wide_roofline(roof: dict, r: dict, D: int, fp32_peak: float, bf16_peak: floa
     direct = uses_direct_form(nd, HYPERS)
     fd1 = descriptor_flops(nd, HYPERS, direct=direct)
     _, tc_pair = algorithmic_flops_per_pair("adjoint", nd=nd, D=D, widths=WIDTHS, hypers=HYPERS)
-    names = (["k_desc_direct_fwd", "k_mlp_grad", "k_desc_direct_bwd"] if direct else
-             ["k_adj_desc (forward)", "k_mlp_grad", "k_adj_desc (backward)"])
+    net = net_kernel(D, WIDTHS, ACT)
+    names = (["k_desc_direct_fwd", net, "k_desc_direct_bwd"] if direct else
+             ["k_adj_desc (forward)", net, "k_adj_desc (backward)"])
     P = r["P"]
     stages = []
     for name, ms, (fl, bound) in zip(names, r["stage_ms"], ((fd1, "fp32"), (tc_pair, "tensor"), (2 * fd1, "fp32"))):
@@ -636,7 +652,9 @@ def run_gpu(args, rank: int, world: int, local_rank: int) -> None:
                       "peak": peaks["bf16_tflops"], "frac_executed": 3.0 * tc_alg / peaks["bf16_tflops"],
                       "note": "net on the tensor cores as three bf16 products per multiply-add (bf16x3)"}
         wide = m == "adjoint" and (max(WIDTHS) > 64 or HYPERS != (10, 8, 4))
-        kernel = {"fd": "k_forces_fd", "fd_split": "k_descriptors + k_mlp + k_fd_scatter"}.get(m, "k_forces_adjoint")
+        split = ("k_descriptors_direct" if uses_direct_form(get_shape(SHAPE).nd, HYPERS) else "k_descriptors") + \
+            " + k_mlp_tiled + k_fd_scatter"
+        kernel = {"fd": "k_forces_fd", "fd_split": split}.get(m, "k_forces_adjoint")
         traffic = DRAM_BYTES_PER_PAIR.get(m)
         roof = {"bound": "fp32", "kernel": kernel, "achieved": achieved, "peak": fp32_peak,
                 "unit": "TFLOP/s", "frac": achieved / fp32_peak,
