@@ -2,8 +2,8 @@
 
 ``System`` owns the state in torch tensors on one GPU and sequences the C-ABI
 calls of one time step exactly as ``Sim.step`` does (``Sim.py:257-285``):
-force pass (pair filter, descriptors, net, forces/torques), then
-``integrate_step_two``, then ``integrate_step_one``; the Verlet list is rebuilt
+force pass (pair filter, descriptors, net, forces/torques), then integrator step
+two and step one (one launch, ``amlp_nvt_step``); the Verlet list is rebuilt
 every ``nlist_every`` steps (100, ``Sim.py:87``). ``run`` replays segments of
 steps as CUDA graphs.
 

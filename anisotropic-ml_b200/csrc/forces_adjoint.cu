@@ -128,23 +128,19 @@ __device__ __forceinline__ void act8(int act, const float *z, float *f, float *d
 //   m = 2: {C_2, S_2} times 1, z, c7      (d/dz: 0, 1, 14 z)
 //   m = 3: {C_3, S_3} times 1, z;  m = 4: {C_4, S_4}
 // The sums over harmonics run on pairs of them (fma.rn.f32x2): two multiply-adds
-// per instruction at the same rate, which keeps the unrolled loops half as long
-// (4.30 -> 4.17 ms at 131,072 cubes).
+// per instruction at the same rate, which keeps the unrolled loops half as long.
 //
-// Both loops are bound by instruction issue: a multiply-add of the 9 x 24 sums
-// (108 per point and half forward, 204 backward) comes with about as many other
-// instructions. Measured with these changes: the fused kernel 5.02 -> 4.20 ms at
-// 131,072 cubes; at 60,001 cylinders the descriptor forward 751 -> 617 us and the
-// backward 1,594 -> 1,160 us. Slower, so not kept: three threads per pair (twelve
-// warps, 4.99 ms), two teams of 64 pairs per CTA in the fused kernel (4.66 ms), the
-// next point's distance and radial functions one iteration ahead.
+// The FP32 pipe bounds both loops, with two warps per scheduler to fill it: a
+// multiply-add of the 9 x 24 sums (108 per point and half forward, 204 backward)
+// comes with about as many others. 131,072 cubes, fused kernel: 4.20 ms (5.02 with
+// halves by index); 60,001 cylinders: descriptor forward 617 us (751), backward
+// 1,160 us (1,594).
 constexpr int kHalfK = 12;  // harmonics per half
 constexpr int kHalfP = kHalfK / 2;
 // Points per iteration of the forward's loop: four overlap one point's chain
-// (load, square root, cosine, recurrences) with another's sums, 669 -> 617 us at
-// 60,001 cylinders; the fused kernel, whose code is longer, is faster with one
-// (4.20 against 4.23 ms at 131,072 cubes). The backward takes two (1,203 -> 1,160 us,
-// 4.27 -> 4.23 ms).
+// (load, square root, cosine, recurrences) with another's sums (60,001 cylinders: 617
+// us against 669 with one); the fused kernel, whose code is longer, is faster with one
+// (131,072 cubes: 4.20 ms against 4.23). The backward takes two (1,160 us against 1,203).
 constexpr int kWideUnroll = 4, kFusedUnroll = 1, kBackwardUnroll = 2;
 
 __host__ __device__ constexpr int half_l(int H, int kk) {
@@ -549,7 +545,7 @@ __device__ __forceinline__ void mma3(uint32_t d_tmem, const char *a_hi, int K, c
 }
 
 // bf16 hi and lo of 8 values, rounded two at a time (one packed conversion per
-// pair, the same round-to-nearest-even values as tc::split_bf16).
+// pair, round to nearest even): hi + lo == v to about 2^-16 relative.
 __device__ __forceinline__ void split8(const float *v, uint4 &hi, uint4 &lo) {
     uint32_t h[4], l[4];
 #pragma unroll
@@ -2062,7 +2058,7 @@ extern "C" amlp_status amlp_adjoint_workspace_bytes(long long cap, size_t *bytes
     return AMLP_OK;
 }
 
-// Body points the harmonic descriptor passes take (at 48, 115 KB of shared memory per block).
+// Body points the harmonic descriptor passes take (at 48, 98 KB of shared memory per block).
 constexpr int kHarmonicMaxPts = 48;
 static size_t wide_desc_smem(int npts) {
     const int rs = 6 * npts + 1 - ((6 * npts) & 1);

@@ -324,11 +324,10 @@ __global__ void __launch_bounds__(kMlpRows) k_mlp(const float *g, long long rows
 // to ten, so that the weights of a warp are the same for its lanes. Per two k, two
 // 16-byte activation loads and five 16-byte loads that broadcast (two columns' weights
 // of two k) feed 80 multiply-adds, issued as 40 pairs of columns, the next two k's
-// operands loading meanwhile. (A warp of 16 x 2 lanes with 8 rows x 5 columns each
-// took half as many again shared-memory wavefronts, 70 % of the SM's rate.)
+// operands loading meanwhile.
 // Each warp stages its own columns' weights, WT[pair of columns][k][2], by cp.async
-// with the lanes along k: one 128-byte line of a row of W per instruction (a k-major
-// layout took four, and a quarter of the kernel's time). Two parts: k < kTSplit of
+// with the lanes along k: one 128-byte line of a row of W per instruction (four in a
+// k-major layout). Two parts: k < kTSplit of
 // the next layer is copied while this layer's second part is multiplied (its first
 // part is free then), the rest while the outputs are written and the next
 // layer's first part is multiplied. Columns past the last are neither copied nor
@@ -336,8 +335,9 @@ __global__ void __launch_bounds__(kMlpRows) k_mlp(const float *g, long long rows
 // inputs, then overwrite them. Each hidden output is bias + sum_k x_k w_k in
 // ascending k, one rounding per multiply-add; the energy (the one-column output
 // layer) is the bias plus the partial sums of 32 groups of threads over k = cg,
-// cg + 32, ... th_C104, 65,536 bodies (1.95 M rows): 7.80 -> 6.40 ms,
-// of which the products take about four fifths at 0.8 of the multiply-add rate.
+// cg + 32, ... Bound by the multiply-add pipe and shared memory's rate (66 and 70 %).
+// th_C104, 65,536 bodies (1.95 M rows): 6.40 ms (7.80 with 8 rows x 5 columns per
+// thread and a k-major layout), the products about four fifths of it.
 constexpr int kTRows = 128, kTThreads = 512, kTMaxW = 160, kTGroups = kTThreads / 16;
 constexpr int kTWarps = kTThreads / 32;
 constexpr int kTMaxP = kTMaxW / kTWarps / 2;  // pairs of columns per thread: 5
@@ -735,7 +735,7 @@ __device__ __forceinline__ void scatter_tile(const float *fd, const int *ij, int
 
 // STAGED: the rotated halves of variants 4..9 are formed once per tile, in the part of bufB
 // that the descriptor stage leaves free, instead of in both passes of every row; the point
-// loop then has no branch on the variant (20,011 cubes of 26 points: 3,578 -> 3,470 us).
+// loop then has no branch on the variant (20,011 cubes of 26 points: 3,470 us against 3,578).
 // Larger clouds, whose copies do not fit there, rotate on the fly. Floats of bufB that the
 // second passes of variants 8 and 9 take, and the most points that fit after them:
 template <class Cfg>
@@ -944,7 +944,7 @@ extern "C" amlp_status amlp_mlp_energy(const float *d_g, long long rows, const a
     if (amax <= kTMaxW) {  // the register-tiled kernel
         if ((st = set_smem(k_mlp_tiled, kTSmem))) return st;
         long long tiles = (rows + kTRows - 1) / kTRows;
-        int grid = (int)std::min<long long>(tiles, kNumSM);  // one CTA per SM (206 KB of shared memory)
+        int grid = (int)std::min<long long>(tiles, kNumSM);  // one CTA per SM (189 KB of shared memory)
         k_mlp_tiled<<<grid, kTThreads, kTSmem, as_stream(stream)>>>(d_g, rows, m, mlp->d_w, d_e);
         return check_launch();
     }

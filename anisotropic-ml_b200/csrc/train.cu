@@ -21,11 +21,12 @@
 // The weights are read through L1 (a warp shares each of them), so that the shared
 // memory holds rows alone: the more rows per tile, the fewer reductions. R is
 // chosen so that the tiles fill whole rounds of the SMs, at most 64.
-// Bound by the L1 that serves both the rows and the weights; the forward and the deltas
-// take four fifths of the time, the gradient products the rest (without them 261 of 355
-// us). 16,384 rows of the 47-150-150-150-150-1 ReLU net: 327 us, 22 TFLOP/s. Before
-// the tiles, 3,254 us: a thread walked one output column over 32 rows with a
-// shared-memory load per multiply-add, and every 32 rows paid one reduction per weight.
+// Bound by latency with four warps per scheduler: the weights' loads (77 % of them hit
+// L1), the barriers between layers and the rows' loads keep the multiply-add pipe at 37 %.
+// The forward and the deltas take about three quarters of the time. 16,384 rows of the
+// 47-150-150-150-150-1 ReLU net: 330 us, 22 TFLOP/s. Before the tiles, 3,254 us: a
+// thread walked one output column over 32 rows with a shared-memory load per
+// multiply-add, and every 32 rows paid one reduction per weight.
 #include <algorithm>
 
 #include "common.cuh"
@@ -58,9 +59,10 @@ __host__ __device__ constexpr int train_ld(int rg) { return 4 * (rg | 1); }
 // columns are consecutive and k's weights are the floats at w + k step (the
 // deltas', one row of W per k). The next four k's weights load while four k's
 // multiply-adds issue, VEC floats to a load (the rows' alignment; without ROWS, 4 columns):
-// at compile time, as the loads' registers decide the loop's. 128-wide layers, 16-byte
-// loads: 686 -> 608 us for 50,021 rows of 47-128-128-128-1; 150-wide, 8-byte ones as
-// before, but without the choice inside the loop: 347 -> 323 us.
+// at compile time, as the loads' registers decide the loop's (at the 128 registers of the
+// block's 512 threads it spills 164 bytes). 50,021 rows of 47-128-128-128-1: 608 us with
+// 16-byte loads, 686 with 8 bytes (4 for the deltas) chosen inside the loop; 16,384 rows of
+// 47-150 x 4-1, whose rows allow 8 bytes: 323 us against 347.
 template <int NC, bool ROWS, int VEC>
 __device__ __forceinline__ void train_product(float2 (&acc)[2][NC], const float *x, int ld, int K, const float *w,
                                               int col, int step) {
