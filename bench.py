@@ -84,31 +84,30 @@ FORCE_CALLS = {"fd": ["amlp_forces_fd"], "adjoint": ["amlp_forces_adjoint"],
                "fd_split": ["amlp_descriptors", "amlp_mlp_energy", "amlp_fd_scatter"]}
 
 
-# DRAM bytes (read + written) per filtered pair of one force launch, from an ncu capture of
-# dram__bytes_read.sum + dram__bytes_write.sum at 32,768 cube26 bodies (436,636 pairs; the kernels'
-# profiles give the command). The traffic grows with the pairs (a capture at 131,072 bodies gave the
-# same bytes per pair), so the roofline's traffic is this figure times the launch's pairs.
-DRAM_BYTES_PER_PAIR = {"adjoint": 5.340928e6 / 436636, "fd": 5.318912e6 / 436636}
+# DRAM bytes (read + written) per filtered pair of one force launch, from ncu captures of
+# dram__bytes_read.sum + dram__bytes_write.sum at 32,768 bodies (cube26 436,6xx pairs, cyl24
+# 381,342; the kernels' profiles give the commands). The traffic grows with the pairs, so the
+# roofline's traffic is this figure times the launch's pairs.
+DRAM_BYTES_PER_PAIR = {"adjoint": 5.329152e6 / 436636, "fd": 5.385728e6 / 436651}
 # The wide path (nets wider than 64) stores each pair's descriptor row, harmonic sums and dE/dg in
-# HBM between its three launches: the sum over k_adj_desc forward, the net kernel and k_adj_desc backward
-# captured at 32,768 cyl24 bodies (381,342 pairs). The per-pair rows do not depend on the shape or the
-# net, so the figure serves every wide workload.
-DRAM_BYTES_PER_PAIR["adjoint_wide"] = (4.141824e6 + 350.520064e6 + 79.480064e6 + 26.586624e6 + 409.184e6
-                                       + 5.303552e6) / 381342
-# Per stage of the wide path, keyed by (kernel, D): ncu dram__bytes_read.sum + dram__bytes_write.sum per
-# pair at 32,768 th_v1 bodies (87,256 pairs; the profiles give the commands). The descriptor rows
-# depend on D, not on the net or the shape.
+# HBM between its three launches: the sum over k_adj_desc forward, the net kernel and k_adj_desc backward.
+# The per-pair rows do not depend on the shape or the net, so the figure serves every wide workload.
+DRAM_BYTES_PER_PAIR["adjoint_wide"] = (4.062720e6 + 349.499392e6 + 79.459840e6 + 28.819200e6 + 409.154048e6
+                                       + 4.407040e6) / 381342
+# Per stage of the wide path, keyed by (kernel, D), per pair: the harmonic-form passes and k_mlp_pair at
+# D = 47 at 32,768 cyl24 bodies, k_mlp_grad at 8,192 tetra16 bodies (944,580 pairs), the others at 32,768
+# th_v1 bodies (87,25x pairs). The rows depend on D, not on the net or the shape; how much of what a
+# kernel writes reaches DRAM before it ends depends on the size.
 STAGE_DRAM_BYTES_PER_PAIR = {
-    # the harmonic-form passes (clouds of more than 12 points), 32,768 cyl24 bodies, 381,342 pairs
-    ("k_adj_desc (forward)", 47): (4.141824e6 + 350.520064e6) / 381342,
-    ("k_adj_desc (backward)", 47): (409.184e6 + 5.303552e6) / 381342,
-    ("k_mlp_grad", 47): 18.56128e6 / 87256,
-    ("k_mlp_grad", 121): (46.54e6 + 0.39e6) / 87257,
-    ("k_mlp_pair", 47): 18.6e6 / 87256,
-    ("k_desc_direct_fwd", 47): 1.64e6 / 87256,
-    ("k_desc_direct_bwd", 47): 19.54e6 / 87256,
-    ("k_desc_direct_fwd", 121): (2.888960e6 + 1.725440e6) / 87257,
-    ("k_desc_direct_bwd", 121): (47.458304e6 + 0.022528e6) / 87257,
+    ("k_adj_desc (forward)", 47): (4.062720e6 + 349.499392e6) / 381342,
+    ("k_adj_desc (backward)", 47): (409.154048e6 + 4.407040e6) / 381342,
+    ("k_mlp_grad", 47): (196.696320e6 + 136.132608e6) / 944580,
+    ("k_mlp_pair", 47): (79.459840e6 + 28.819200e6) / 381342,
+    ("k_mlp_pair", 121): (46.561792e6 + 2.592000e6) / 87257,
+    ("k_desc_direct_fwd", 47): 1.634048e6 / 87256,
+    ("k_desc_direct_bwd", 47): 19.528448e6 / 87256,
+    ("k_desc_direct_fwd", 121): (1.641216e6 + 0.631296e6) / 87257,
+    ("k_desc_direct_bwd", 121): (47.457024e6 + 0.013824e6) / 87257,
 }
 
 
