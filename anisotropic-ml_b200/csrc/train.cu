@@ -34,7 +34,13 @@
 namespace amlp {
 namespace {
 
-constexpr int kTrainThreads = 512;
+constexpr int kTrainThreads = 512;       // threads per block, one block per SM
+// Nets whose inputs and layers are at most 16 wide take four blocks of 128 threads: their tiles
+// are barriers and latency, which other blocks' tiles fill. 300,000 rows of 1-3-1 (ReLU): 89
+// us, with one block of 512 threads 257, 170 before the tiles; 8-16-16-1: 144 against 404. With 47
+// inputs the blocks gain less, and at 1,000 rows (47-16-1) they lose, 14.4 us against 12.3.
+constexpr int kTrainSmallThreads = 128;
+constexpr int kTrainSmallWidth = 16;
 constexpr int kTrainMaxRows = 64;
 constexpr int kTrainMaxWidth = 256;
 constexpr size_t kTrainSmem = 226 * 1024;
@@ -267,9 +273,9 @@ __device__ __forceinline__ void train_store_delta(const TrainNet &net, const Tra
 // deltas 4; with all lanes along k, the same 40 multiply-adds took 21 wavefronts instead
 // of 9 and the shared memory bounded them (47-128-128-128-1, 50,021 rows: 608 -> 589 us;
 // the reductions, in 32-byte pieces now, cost the 150-wide net 1 %).
-template <int NI, int NJ>
+template <int NT, int NI, int NJ>
 __device__ __forceinline__ void train_weights(const TrainNet &net, const TrainTile &t, float *grad, int L) {
-    constexpr int nw = kTrainThreads / 32;
+    constexpr int nw = NT / 32;
     const int K = net.dims[L], N = net.dims[L + 1], ld = net.ld, R = 4 * net.rg;
     const int lane = t.tid & 31, nkb = (K + 8 * NI - 1) / (8 * NI), nnb = (N + 4 * NJ - 1) / (4 * NJ);
     float *gW = grad + net.woff[L];
@@ -315,17 +321,19 @@ __device__ __forceinline__ void train_weights(const TrainNet &net, const TrainTi
 }
 
 // Multiply-adds per lane and row of a layer's tiles: whole rounds of the warps.
+template <int NT>
 __device__ __forceinline__ int train_tile_cost(int N, int K, int NI, int NJ) {
     const int tiles = ((K + 8 * NI - 1) / (8 * NI)) * ((N + 4 * NJ - 1) / (4 * NJ));
-    constexpr int nw = kTrainThreads / 32;
+    constexpr int nw = NT / 32;
     return (tiles + nw - 1) / nw * NI * NJ;
 }
 
 // dL/db of layer L.
+template <int NT>
 __device__ __forceinline__ void train_bias(const TrainNet &net, const TrainTile &t, float *grad, int L) {
     const int K = net.dims[L], N = net.dims[L + 1], ld = net.ld, R = 4 * net.rg;
     float *gb = grad + net.woff[L] + (size_t)N * K;
-    for (int n = t.tid; n < N; n += kTrainThreads) {
+    for (int n = t.tid; n < N; n += NT) {
         const float *d = t.sm + (net.feat[L + 1] + n) * ld;
         float s = 0.f;
         for (int r = 0; r < R; r += 4) {
@@ -336,15 +344,16 @@ __device__ __forceinline__ void train_bias(const TrainNet &net, const TrainTile 
     }
 }
 
-__global__ void __launch_bounds__(kTrainThreads, 1) k_mlp_loss_grad(const float *g, const float *y, const float *dy,
-                                                                    long long rows, TrainNet net, const float *w,
-                                                                    float *grad, double *loss) {
+template <int NT>
+__global__ void __launch_bounds__(NT, kTrainThreads / NT) k_mlp_loss_grad(const float *g, const float *y,
+                                                                         const float *dy, long long rows, TrainNet net,
+                                                                         const float *w, float *grad, double *loss) {
     extern __shared__ __align__(16) float sm[];
     const int ld = net.ld, R = 4 * net.rg;
     TrainTile t;
     t.sm = sm;
     t.tid = threadIdx.x;
-    t.ncg = kTrainThreads / net.rg;
+    t.ncg = NT / net.rg;
     t.cg = t.tid / net.rg;
     t.rg = t.tid - t.cg * net.rg;
     t.on = t.cg < t.ncg;
@@ -353,7 +362,7 @@ __global__ void __launch_bounds__(kTrainThreads, 1) k_mlp_loss_grad(const float 
         const int nr = t.nr = (int)min((long long)R, rows - r0);
         const int D = net.dims[0];
         // the tile's descriptor rows, a warp per row (coalesced); rows past the end are zero
-        for (int r = t.tid >> 5; r < R; r += kTrainThreads / 32)
+        for (int r = t.tid >> 5; r < R; r += NT / 32)
             for (int d = t.tid & 31; d < D; d += 32) sm[d * ld + r] = r < nr ? g[(r0 + r) * D + d] : 0.f;
         __syncthreads();
         for (int L = 0; L < net.n_layers; ++L) {
@@ -394,14 +403,14 @@ __global__ void __launch_bounds__(kTrainThreads, 1) k_mlp_loss_grad(const float 
         for (int L = net.n_layers - 1; L >= 0; --L) {
             const int K = net.dims[L], N = net.dims[L + 1];
             // the tile with which the layer's tiles cost the warps least
-            const int c55 = train_tile_cost(N, K, 5, 5), c54 = train_tile_cost(N, K, 5, 4);
-            const int c44 = train_tile_cost(N, K, 4, 4), c34 = train_tile_cost(N, K, 3, 4);
+            const int c55 = train_tile_cost<NT>(N, K, 5, 5), c54 = train_tile_cost<NT>(N, K, 5, 4);
+            const int c44 = train_tile_cost<NT>(N, K, 4, 4), c34 = train_tile_cost<NT>(N, K, 3, 4);
             const int least = min(min(c55, c54), min(c44, c34));
-            if (c55 == least) train_weights<5, 5>(net, t, grad, L);
-            else if (c54 == least) train_weights<5, 4>(net, t, grad, L);
-            else if (c44 == least) train_weights<4, 4>(net, t, grad, L);
-            else train_weights<3, 4>(net, t, grad, L);
-            train_bias(net, t, grad, L);
+            if (c55 == least) train_weights<NT, 5, 5>(net, t, grad, L);
+            else if (c54 == least) train_weights<NT, 5, 4>(net, t, grad, L);
+            else if (c44 == least) train_weights<NT, 4, 4>(net, t, grad, L);
+            else train_weights<NT, 3, 4>(net, t, grad, L);
+            train_bias<NT>(net, t, grad, L);
             if (L == 0) break;
             const int nc = train_columns(K, t.ncg), k0 = t.cg * nc;
             const bool mine = t.on && k0 < K;
@@ -468,22 +477,28 @@ static amlp_status launch_grad(const float *d_g, const float *d_y, const float *
         net.woff[k] = off;
         off += (long long)mlp->dims[k + 1] * mlp->dims[k] + mlp->dims[k + 1];
     }
+    int wide = 0;
+    for (int k = 0; k < mlp->n_layers; ++k) wide = std::max(wide, mlp->dims[k]);
+    const bool small = wide <= kTrainSmallWidth;
+    const int blocks = small ? kNumSM * (kTrainThreads / kTrainSmallThreads) : kNumSM;  // running at once
+    const size_t room = small ? kTrainSmem / (kTrainThreads / kTrainSmallThreads) : kTrainSmem;
     // Rows per tile: as many as the shared memory holds, at most 64, then the fewest
-    // (a multiple of 4) with which the tiles make as few rounds of the SMs
+    // (a multiple of 4) with which the tiles make as few rounds of the blocks
     int rg = kTrainMaxRows / 4;
-    while (rg > 1 && (size_t)feat * train_ld(rg) * sizeof(float) > kTrainSmem) --rg;
-    const long long rounds = (rows + (long long)kNumSM * 4 * rg - 1) / ((long long)kNumSM * 4 * rg);
-    const long long per = (rows + kNumSM * rounds - 1) / (kNumSM * rounds);
+    while (rg > 1 && (size_t)feat * train_ld(rg) * sizeof(float) > room) --rg;
+    const long long rounds = (rows + (long long)blocks * 4 * rg - 1) / ((long long)blocks * 4 * rg);
+    const long long per = (rows + blocks * rounds - 1) / (blocks * rounds);
     rg = (int)std::min<long long>(rg, std::max<long long>(1, (per + 3) / 4));
     net.rg = rg;
     net.ld = train_ld(rg);
     const size_t smem = (size_t)feat * net.ld * sizeof(float);
-    if (smem > kTrainSmem) return AMLP_ERR_UNSUPPORTED;
-    AMLP_CHECK_CUDA(cudaFuncSetAttribute(k_mlp_loss_grad, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    if (smem > room) return AMLP_ERR_UNSUPPORTED;
+    const auto kern = small ? k_mlp_loss_grad<kTrainSmallThreads> : k_mlp_loss_grad<kTrainThreads>;
+    AMLP_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     const long long tiles = (rows + 4 * rg - 1) / (4 * rg);
-    const int grid = (int)std::min<long long>(tiles, kNumSM);
-    k_mlp_loss_grad<<<grid, kTrainThreads, smem, as_stream(stream)>>>(d_g, d_y, d_dy, rows, net, mlp->d_w, d_grad,
-                                                                      d_dy ? nullptr : d_loss);
+    const int grid = (int)std::min<long long>(tiles, blocks);
+    kern<<<grid, small ? kTrainSmallThreads : kTrainThreads, smem, as_stream(stream)>>>(
+        d_g, d_y, d_dy, rows, net, mlp->d_w, d_grad, d_dy ? nullptr : d_loss);
     return check_launch();
 }
 
