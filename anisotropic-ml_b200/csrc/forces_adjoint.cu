@@ -1498,8 +1498,9 @@ __global__ void __launch_bounds__(kMThreads, 1) k_mlp_grad(const float *g_rows, 
 //    epilogues, the 30 MMAs of a 160-wide layer took 3.9 k cycles to issue and 2.4 k to run.
 //  - The warp before it copies the next layer's weights when both products are complete (wfree).
 //  - A team without a tile (last round) is left out of the round.
-//  - A role whose wait gives up sets `quit` and leaves; the others follow, the products in
-//    flight are drained, and the block's rows are zeroed (drop_rows).
+//  - A role whose wait gives up sets `quit` and leaves; the others follow (pair_wait, or at
+//    worst their own limit), the products in flight are drained, and the block's rows are
+//    zeroed (drop_rows).
 // Two 160-wide operand tiles and a layer's weights do not fit shared memory: with TMEM_A
 // the first team's operand tile is in TMEM (bf16 pairs, hi and lo), which ReLU leaves
 // room for (its derivatives are bits in registers). Smooth activations take this kernel
